@@ -85,12 +85,15 @@ __device__ void build_head_tables(HeadTables& ht, const float* cb_global, int la
         __syncwarp();
         return;
     }
-    // thresholds: bisection between cb[c-1] (code c-1) and cb[c] (code c)
+    // thresholds: bisection between cb[c-1] (code c-1) and cb[c] (code c).  Inside that bracket the nearest of the levels
+    // 0..c-1 is c-1 and the nearest of the levels c..15 is c (fp32 rounding is monotone), so "code >= c" is one strict
+    // comparison of two distances instead of the 16-level scan.
     if (lane >= 1 && lane < 16) {
         int lo = order_key(c_prev), hi = order_key(c_me);
         while ((int64_t)hi - lo > 1) {
             const int mid = (int)(((int64_t)lo + hi) >> 1);
-            if (code_by_scan(order_unkey(mid), ht.cb) >= lane) hi = mid; else lo = mid;
+            const float y = order_unkey(mid);
+            if (fabsf(__fsub_rn(y, c_me)) < fabsf(__fsub_rn(y, c_prev))) hi = mid; else lo = mid;
         }
         ht.thr[lane] = order_unkey(hi);
     }
@@ -349,13 +352,35 @@ __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(FastQua
                              kFqWarps * kStageBytesPerWarp + warp * kBallotBytesPerWarp;
     const uint32_t my_ballots = ballots + (uint32_t)(t * 4 + (g & 1) * 2) * 4;
 
-    for (int h = warp; h < n_tabs; h += kFqWarps) build_head_tables(tabs[h], a.codebooks + h * 16, lane);
+    // The 8-token groups of all (user, head) pairs, in order, are dealt out in equal consecutive shares, one per warp of the
+    // grid: a warp's share may begin and end inside a pair.  A whole pair per warp left the last round of a large call
+    // mostly empty and all but 8 warps of a one-user call idle: K and V of 1,024 users x 8 heads x 256 tokens (3.46 pairs
+    // per warp, so 4 rounds) 989 us against 862 us now, 256 x 8 x 203 fp32 rows with their rotation 202 against 187 us.
+    const int T = (int)a.T;                                          // fast_quantize_eligible: groups and tokens fit 32 bits
+    const uint32_t gpp = (uint32_t)(T + 7) >> 3;                     // groups of one pair
+    uint32_t gi, last;
+    {
+        const uint64_t n_groups = (uint64_t)(a.B * a.H) * gpp, n_warps = (uint64_t)gridDim.x * kFqWarps;
+        const uint64_t wid = (uint64_t)blockIdx.x * kFqWarps + warp, w0 = wid - warp;
+        gi = (uint32_t)(n_groups * wid / n_warps);
+        last = (uint32_t)(n_groups * (wid + 1) / n_warps);
+        // the codebooks of the heads this block's shares touch
+        const uint64_t p0 = n_groups * w0 / n_warps / gpp, p1 = (n_groups * (w0 + kFqWarps) / n_warps + gpp - 1) / gpp;
+        const int need = a.cb_per_head ? (p1 - p0 < (uint64_t)a.H ? (int)(p1 - p0) : a.H) : (p1 > p0);
+        for (int i = warp; i < need; i += kFqWarps) {
+            const int h = a.cb_per_head ? (int)((p0 + i) % a.H) : 0;
+            build_head_tables(tabs[h], a.codebooks + h * 16, lane);
+        }
+    }
     __syncthreads();
 
-    const int64_t n_pairs = a.B * a.H;
-    for (int64_t p = (int64_t)blockIdx.x * kFqWarps + warp; p < n_pairs; p += (int64_t)gridDim.x * kFqWarps) {
-        const int64_t b = p / a.H;
-        const int h = (int)(p % a.H);
+    while (gi < last) {
+        const uint32_t p = gi / gpp;
+        const int t_begin = (int)(gi - p * gpp) * 8;
+        const int t_end = (last - gi) < gpp && (int)(t_begin + (last - gi) * 8) < T ? (int)(t_begin + (last - gi) * 8) : T;
+        gi = (p + 1) * gpp;
+        const int64_t b = p / (uint32_t)a.H;
+        const int h = (int)(p % (uint32_t)a.H);
         const int32_t uid = a.user_ids ? a.user_ids[b] : a.user_id;
         const int seed = seed_of(uid, h);
         const uint32_t* grow = a.g_rows + (size_t)seed * kQjlDim * 4;
@@ -376,19 +401,19 @@ __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(FastQua
         const int64_t out_base = b * a.os_b + (int64_t)h * a.os_h + (a.out_offsets ? a.out_offsets[b] : a.out_offset);
 
         // rows past the end of a group are clamped to the last token (computed, never stored)
-        if (a.T > 0) stage_row<DT>(stage, a.x, in_base + (g < a.T ? g : a.T - 1) * a.xs_t);
-        for (int64_t t0 = 0; t0 < a.T; t0 += 8) {
-            const int64_t tr = t0 + g;
-            const bool active = tr < a.T;
+        stage_row<DT>(stage, a.x, in_base + (t_begin + g < T ? t_begin + g : T - 1) * a.xs_t);
+        for (int t0 = t_begin; t0 < t_end; t0 += 8) {
+            const int tr = t0 + g;
+            const bool active = tr < T;
             cp_async_wait_all();
             float y[32];
             {
                 uint4 c[Row32<DT>::kChunks];
 #pragma unroll
                 for (int k = 0; k < Row32<DT>::kChunks; ++k) c[k] = lds_u4(stage + k * 512);
-                if (t0 + 8 < a.T) {                 // the chunks are in registers: refill the buffer with the next group
-                    const int64_t tn = t0 + 8 + g;
-                    stage_row<DT>(stage, a.x, in_base + (tn < a.T ? tn : a.T - 1) * a.xs_t);
+                if (t0 + 8 < t_end) {               // the chunks are in registers: refill the buffer with the next group
+                    const int tn = tr + 8;
+                    stage_row<DT>(stage, a.x, in_base + (tn < T ? tn : T - 1) * a.xs_t);
                 }
                 Row32<DT>::unpack(c, y);
             }
@@ -624,7 +649,8 @@ bool fast_quantize_eligible(const FastQuantArgs& a, int dtype) {
     if (!fq_aligned(a.x, 16) || a.xs_b % vec || a.xs_h % vec || a.xs_t % vec) return false;
     if (!fq_aligned(a.nib, 16) || !fq_aligned(a.qjl, 2)) return false;
     if ((a.qjl == nullptr) != (a.norms == nullptr)) return false;
-    return a.T > 0;
+    // token and group numbers of the kernel are 32-bit (every row's packed bytes would not fit a GPU's memory sooner)
+    return a.T > 0 && a.T <= 0x7ffffff0LL && a.B * a.H * ((a.T + 7) >> 3) < 0xffffffffLL;
 }
 
 template <int DT>
@@ -635,9 +661,9 @@ static int32_t launch_fast_t(const FastQuantArgs& a, int rotate, cudaStream_t st
     const int n_tabs = a.cb_per_head ? a.H : 1;
     const size_t smem = sizeof(HeadTables) * n_tabs + (size_t)kFqWarps * 16 * 32 * sizeof(uint4) +
                         (size_t)kFqWarps * (kStageBytesPerWarp + kBallotBytesPerWarp);
-    const int64_t pairs = a.B * a.H;
-    int64_t blocks = (pairs + kFqWarps - 1) / kFqWarps;
-    if (blocks > 2 * sms) blocks = 2 * sms;
+    const int64_t groups = a.B * a.H * ((a.T + 7) >> 3);
+    // two resident CTAs per SM; fewer groups than warps are spread over the SMs, one group per warp
+    const int64_t blocks = groups < 2 * sms ? groups : 2 * sms;
     const bool signs = a.qjl != nullptr;
     auto kern = signs ? (rotate ? fast_quantize_kernel<DT, true, true> : fast_quantize_kernel<DT, false, true>)
                       : (rotate ? fast_quantize_kernel<DT, true, false> : fast_quantize_kernel<DT, false, false>);
