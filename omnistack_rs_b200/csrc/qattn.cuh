@@ -47,8 +47,8 @@ struct AttnArgs {
 // The tensor-core kernel dequantises through a table of fp16 centroid pairs.  fp16 rounds a centroid by at most
 // 2^-9 = 1.95e-3 while |c| < 8 (1e-3 below 4, where Lloyd-Max codebooks of rotated unit-variance data lie) and by
 // up to 3.9e-3 from 8 on, which a 3e-3 output budget cannot absorb; codebooks with a centroid of magnitude 8 or
-// more, infinite or NaN ("wide") are served by the fp32 lane-per-key kernel instead.  Both kernels evaluate this
-// same predicate on the device (over every codebook of the call), so the choice needs no host copy and cannot go
+// more, infinite or NaN ("wide") are served by the fp32 lane-per-key code instead.  The kernels evaluate this
+// predicate on the device (over every codebook of the call), so the choice needs no host copy and cannot go
 // stale.
 constexpr float kFp16CentroidLimit = 8.0f;
 __device__ __forceinline__ bool centroid_is_wide(float c) { return !(fabsf(c) < kFp16CentroidLimit); }

@@ -30,6 +30,7 @@
 // Work distribution.  Persistent grid, one CTA per SM.  Calls without key splits assign items statically (equal
 // sizes); split-K calls draw tickets from a counter in the workspace so ragged cache lengths stay balanced.
 #include "qattn.cuh"
+#include "qattn_lane.cuh"
 #include <cuda.h>
 #include <mutex>
 #include <utility>
@@ -680,9 +681,15 @@ __device__ __forceinline__ void ring_consumed(Ring& r) {
     --r.in_flight;
 }
 
+// Out of line: inlined, its 128 accumulators would take part in the register allocation of the main loop.
+template <int DT>
+__device__ __noinline__ void serve_in_fp32(const AttnArgs& a, LaneScratch& sc, int64_t first, int64_t stride) {
+    lane_per_key_rows<DT>(a, sc, first, stride);
+}
+
 template <int DT, bool QJL, bool ONECOL, bool VPAIR, bool LORA>
 __global__ void __launch_bounds__(kMmaWarps * 32, 1)
-qattn_mma_kernel(AttnArgs a, int64_t n_items, const __grid_constant__ CUtensorMap map_k,
+qattn_mma_kernel(const __grid_constant__ AttnArgs a, int64_t n_items, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -700,12 +707,15 @@ qattn_mma_kernel(AttnArgs a, int64_t n_items, const __grid_constant__ CUtensorMa
     const uint32_t my_off = (uint32_t)warp < n_front ? (uint32_t)warp * kWarpBlockBytes
                                                      : lut_off + kLutSpan + ((uint32_t)warp - n_front) * kWarpBlockBytes;
     {
-        // a codebook the fp16 table cannot hold to the error budget: the whole grid stands down (the same test in
-        // the lane-per-key kernel, launched behind this one, makes that kernel serve the call)
+        // a codebook the fp16 table cannot hold to the error budget: the whole grid serves the call in fp32 instead
         const int n_cb = a.cb_per_head ? a.Hkv * 16 : 16;
         bool wide = false;
         for (int i = threadIdx.x; i < n_cb; i += blockDim.x) wide = wide || centroid_is_wide(__ldg(a.codebooks + i));
-        if (__syncthreads_or(wide)) return;
+        if (__syncthreads_or(wide)) {
+            const int64_t cta = blockIdx.x + (int64_t)gridDim.x * blockIdx.y, ctas = (int64_t)gridDim.x * gridDim.y;
+            serve_in_fp32<DT>(a, reinterpret_cast<LaneScratch*>(smem)[warp], cta * kMmaWarps + warp, ctas * kMmaWarps);
+            return;
+        }
     }
     const float lut_scale = lut_scale_of(a.codebooks + (a.cb_per_head ? cb_head * 16 : 0));
     const float inv_lut = 1.f / lut_scale;
@@ -1071,7 +1081,8 @@ static int32_t allow_full_smem(const void* kern, int dev) {
 }
 
 template <int DT>
-static int32_t launch_mma_t(const AttnArgs& a, cudaStream_t st) {
+static int32_t launch_mma_t(const AttnArgs& args, cudaStream_t st) {
+    AttnArgs a = args;
     int dev = 0, sms = 148;
     OMNI_CUDA(cudaGetDevice(&dev));
     int32_t rc = sm_count_of(dev, &sms);
@@ -1082,8 +1093,6 @@ static int32_t launch_mma_t(const AttnArgs& a, cudaStream_t st) {
     int64_t items, ctas;
     unsigned gy;
     const int64_t n_ctiles = ((int64_t)(a.Hq / a.Hkv) * a.T + 7) / 8;
-    // ticket counters: cleared by the preparation launch when there is one, by a memset node otherwise
-    if (a.work_counter && !a.qprep) OMNI_CUDA(cudaMemsetAsync(a.work_counter, 0, kWorkCounterBytes, st));
     if (a.cb_per_head) {
         items = a.B * a.n_splits * n_ctiles;
         ctas = sms / a.Hkv > 0 ? sms / a.Hkv : 1;
@@ -1094,6 +1103,10 @@ static int32_t launch_mma_t(const AttnArgs& a, cudaStream_t st) {
         gy = 1;
     }
     if (ctas > items) ctas = items;                 // few items: one per CTA, spread over the SMs
+    // ticket counters: not needed when every item has a warp of its own; cleared by the preparation launch when there is
+    // one, by a memset node otherwise
+    if (items <= ctas * kMmaWarps) a.work_counter = nullptr;
+    if (a.work_counter && !a.qprep) OMNI_CUDA(cudaMemsetAsync(a.work_counter, 0, kWorkCounterBytes, st));
     dim3 grid((unsigned)ctas, gy);
     CUtensorMap map_k, map_v;
     rc = make_nibble_map(&map_k, a.k_nib);
