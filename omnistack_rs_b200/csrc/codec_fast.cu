@@ -561,15 +561,39 @@ __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(FastQua
                 }
                 uint32_t amb16 = every_fourth_bit(wa0, sh) | (every_fourth_bit(wa1, sh) << 8);
                 if (!active) amb16 = 0u;
-                // ---- exact recomputation of the undecided projections, one per row at a time --------------
+                // ---- recomputation of the undecided projections, one per row at a time.  First in fp32: four running sums of
+                // eight signed residuals each, added up over the row's lanes, are off by at most 12 roundings of partial sums
+                // no larger than 128 emax, 12 * 2^-24 * 128 emax < 1e-4 emax, so a larger result has the exact sum's sign; the
+                // few that are not (3 in 64 of the undecided), and rows that could not be scaled, go to fp64.  (Every undecided
+                // projection in fp64, a chain of 32 conversions and adds: prefill of 1,024 users x 8 heads x 256 tokens 862 us
+                // against 842 us.)
                 uint64_t pending = (uint64_t)__shfl_sync(kFullMask, amb16, 4 * g) |
                                    ((uint64_t)__shfl_sync(kFullMask, amb16, 4 * g + 1) << 16) |
                                    ((uint64_t)__shfl_sync(kFullMask, amb16, 4 * g + 2) << 32) |
                                    ((uint64_t)__shfl_sync(kFullMask, amb16, 4 * g + 3) << 48);
+                const float sure = degenerate ? INFINITY : emax * 1e-4f;
+                uint64_t close = 0ull;
                 while (__any_sync(kFullMask, pending != 0ull)) {
                     const bool have = pending != 0ull;
                     const int pi = have ? __ffsll((long long)pending) - 1 : 0;
                     if (have) pending &= pending - 1ull;
+                    const uint32_t flip = ~__ldg(grow + pi * 4 + t);
+                    float p[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) p[i & 3] += __uint_as_float(__float_as_uint(y[i]) ^ ((flip << (31 - i)) & 0x80000000u));
+                    float acc = (p[0] + p[1]) + (p[2] + p[3]);
+                    acc += __shfl_xor_sync(kFullMask, acc, 1);
+                    acc += __shfl_xor_sync(kFullMask, acc, 2);
+                    if (have && !(fabsf(acc) > sure)) close |= 1ull << pi;
+                    if (have && t == (pi >> 4)) {
+                        const uint32_t m = 1u << (pi & 15);
+                        bits16 = (acc >= 0.f) ? (bits16 | m) : (bits16 & ~m);
+                    }
+                }
+                while (__any_sync(kFullMask, close != 0ull)) {
+                    const bool have = close != 0ull;
+                    const int pi = have ? __ffsll((long long)close) - 1 : 0;
+                    if (have) close &= close - 1ull;
                     const uint32_t gw = __ldg(grow + pi * 4 + t);
                     double acc = 0.0;
 #pragma unroll
