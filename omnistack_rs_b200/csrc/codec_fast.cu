@@ -617,11 +617,49 @@ __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(FastQua
     }
 }
 
-// Stand-alone rotation with the same row layout (8 rows per warp, 4 lanes per row, 16-byte loads and stores): two
-// cross-lane stages instead of five, which matters for 16-bit rows, where the warp-per-row kernel is bound by
-// shuffle throughput.
+// The same transform of a row whose 16-byte chunks are dealt to its four lanes in turn: chunk 4 m + t is y[E m .. E m + E - 1]
+// of lane t (E elements per chunk), so the stages below E are inside the thread, the next two across lanes and the rest
+// inside the thread again -- the reference's order h = 1 .. 64, one rounding per add / subtract.
+template <int E>
+__device__ __forceinline__ void rotate_row32_chunked(float (&y)[32], int t) {
+    auto stage = [&](int hh) {                                    // elements i and i + 16 as packed pairs
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            if ((i & hh) == 0) {
+                const float u0 = y[i], u1 = y[i + 16], v0 = y[i | hh], v1 = y[(i | hh) + 16];
+                add2(y[i], y[i + 16], u0, u1, v0, v1);
+                fma2(y[i | hh], y[(i | hh) + 16], v0, v1, -1.f, -1.f, u0, u1);
+            }
+        }
+    };
+#pragma unroll
+    for (int hh = 1; hh < E; hh <<= 1) stage(hh);
+#pragma unroll
+    for (int m = 1; m <= 2; m <<= 1) {
+        const float sgn = (t & m) ? -1.f : 1.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const float o0 = __shfl_xor_sync(kFullMask, y[i], m), o1 = __shfl_xor_sync(kFullMask, y[i + 16], m);
+            fma2(y[i], y[i + 16], sgn, sgn, y[i], y[i + 16], o0, o1);
+        }
+    }
+#pragma unroll
+    for (int hh = E; hh < 16; hh <<= 1) stage(hh);
+    const float sc = __uint_as_float(OMNI_WHT_SCALE_BITS);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+        const float u = y[i], v = y[i + 16];
+        mul2(y[i], y[i + 16], __fadd_rn(u, v), __fsub_rn(u, v), sc, sc);
+    }
+}
+
+// Stand-alone rotation, 8 rows per warp, 4 lanes per row: two cross-lane stages instead of five, which matters for 16-bit
+// rows, where the warp-per-row kernel is bound by shuffle throughput.  A row's lanes take its 16-byte chunks in turn, so an
+// access of the warp touches 64 consecutive bytes of each row (with 64 consecutive bytes per LANE it touched 16 lines for
+// the same 512 bytes and L1 was the limit: 1,048,576 bf16 rows 107 us against 85 us, 94 % of the copy peak).
 template <int DT>
 __global__ void __launch_bounds__(kFqWarps * 32) fast_rotate_kernel(const void* x, void* y_out, int64_t n_rows) {
+    constexpr int kChunks = Row32<DT>::kChunks, E = 32 / kChunks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
     const int64_t n_groups = (n_rows + 7) / 8;
@@ -629,18 +667,18 @@ __global__ void __launch_bounds__(kFqWarps * 32) fast_rotate_kernel(const void* 
         const int64_t row = grp * 8 + g;
         const bool active = row < n_rows;
         const int64_t rc = active ? row : n_rows - 1;
-        uint4 c[Row32<DT>::kChunks];
-        const uint4* src = reinterpret_cast<const uint4*>(Row32<DT>::addr(x, rc * kHeadDim + 32 * t));
+        uint4 c[kChunks];
+        const uint4* src = reinterpret_cast<const uint4*>(Row32<DT>::addr(x, rc * kHeadDim)) + t;
 #pragma unroll
-        for (int k = 0; k < Row32<DT>::kChunks; ++k) c[k] = __ldg(src + k);
+        for (int k = 0; k < kChunks; ++k) c[k] = __ldg(src + 4 * k);
         float y[32];
         Row32<DT>::unpack(c, y);
-        rotate_row32(y, t);
+        rotate_row32_chunked<E>(y, t);
         Row32<DT>::pack(y, c);
         if (active) {
-            uint4* dst = reinterpret_cast<uint4*>(const_cast<char*>(Row32<DT>::addr(y_out, rc * kHeadDim + 32 * t)));
+            uint4* dst = reinterpret_cast<uint4*>(const_cast<char*>(Row32<DT>::addr(y_out, rc * kHeadDim))) + t;
 #pragma unroll
-            for (int k = 0; k < Row32<DT>::kChunks; ++k) dst[k] = c[k];
+            for (int k = 0; k < kChunks; ++k) dst[4 * k] = c[k];
         }
     }
 }
