@@ -127,6 +127,15 @@ int32_t omni_lloyd_max_fit(const float* sorted, int64_t n_total, const int64_t* 
                            int32_t max_iters, double tol, void* workspace, size_t workspace_bytes,
                            float* codebooks, int32_t* iters_out, void* stream);
 
+/* Ascending fp32 order within every group (what omni_lloyd_max_fit expects): NaN last, -0 before +0.  Groups lie back to
+ * back in `samples`; group_offsets: device int64 [n_groups+1] as above, no group empty; chunk_base: device int64
+ * [n_groups+1], the running sum of ceil(size of group / OMNI_SORT_CHUNK), n_chunks its last entry.  `sorted` must not
+ * alias `samples`; `workspace`: device scratch of omni_sort_groups_workspace_bytes(...) bytes.  n_total < 2^31.       */
+#define OMNI_SORT_CHUNK 4096
+size_t  omni_sort_groups_workspace_bytes(int64_t n_total, int32_t n_groups, int64_t n_chunks);
+int32_t omni_sort_groups(const float* samples, int64_t n_total, const int64_t* group_offsets, const int64_t* chunk_base,
+                         int32_t n_groups, int64_t n_chunks, void* workspace, size_t workspace_bytes, float* sorted, void* stream);
+
 /* Row-seeded codec (kernels/quantize.py:456-499 `quantize_rows`, :502-537
  * `dequantize_rows`): row i of n_rows contiguous fp32 rows uses seed
  * (user_id mod 1024) xor (base_head_idx + i), for any non-negative row key base_head_idx + i below 2^31 (the

@@ -5,11 +5,14 @@ Mirrors ``omnistack_rs/quantization/codebook.py`` of the reference (``LloydMaxCa
 and algorithm (equal-mass initialisation, first-index nearest-centroid assignment, mean
 update, empty cells stay put, stop below ``convergence_tol``, sorted float32 output).
 
-The fit itself is ``omni_lloyd_max_fit``: the samples are sorted once on the device, and the whole
+The fit itself is ``omni_lloyd_max_fit``: the samples of all groups are sorted once on the device
+(``omni_sort_groups``), and the whole
 iteration then runs in one kernel launch on cell boundaries and prefix sums (all groups of
 ``calibrate_per_group`` in the same launch).  There is no host implementation.
 """
 from __future__ import annotations
+
+from itertools import accumulate
 
 import torch
 
@@ -18,6 +21,7 @@ from .. import _lib
 N_CENTROIDS: int = 16
 _DEFAULT_MAX_ITERS: int = 300
 _DEFAULT_TOL: float = 1e-6
+_SORT_CHUNK: int = 4096                      # OMNI_SORT_CHUNK of the C header
 
 
 class LloydMaxCalibrator:
@@ -65,12 +69,23 @@ def _fit_groups(groups, max_iters: int, tol: float) -> torch.Tensor:
     for n in sizes:
         if n < N_CENTROIDS:
             raise ValueError(f"Need at least {N_CENTROIDS} samples; got {n}")
-    ordered = torch.cat([g.sort().values for g in groups]) if len(groups) > 1 else groups[0].sort().values
-    offsets = torch.tensor([0] + sizes, dtype=torch.int64).cumsum(0).to(dev)
-    total = sum(sizes)
-    ws_bytes = lib.omni_lloyd_max_workspace_bytes(total)
-    ws = torch.empty(ws_bytes // 8, dtype=torch.float64, device=dev)
-    out = torch.empty(len(groups), N_CENTROIDS, dtype=torch.float32, device=dev)
+    total, n = sum(sizes), len(groups)
+    chunks = [-(-s // _SORT_CHUNK) for s in sizes]
+    table = torch.tensor([list(accumulate(sizes, initial=0)), list(accumulate(chunks, initial=0))], dtype=torch.int64).to(dev)
+    offsets, chunk_base, n_chunks = table[0], table[1], sum(chunks)
+    own_sort = total < 1 << 31
+    sort_bytes = lib.omni_sort_groups_workspace_bytes(total, n, n_chunks) if own_sort else 0
+    ws_bytes = max(lib.omni_lloyd_max_workspace_bytes(total), sort_bytes)
+    ws = torch.empty(-(-ws_bytes // 8), dtype=torch.float64, device=dev)
+    out = torch.empty(n, N_CENTROIDS, dtype=torch.float32, device=dev)
+    if own_sort:
+        flat = torch.cat(groups) if n > 1 else groups[0].contiguous()
+        ordered = torch.empty(total, dtype=torch.float32, device=dev)
+        with _lib.on_device(dev):
+            _lib.check(lib.omni_sort_groups(_lib.ptr(flat), total, _lib.ptr(offsets), _lib.ptr(chunk_base), n, n_chunks, _lib.ptr(ws), ws_bytes,
+                                            _lib.ptr(ordered), _lib.stream_ptr(dev)))
+    else:                                              # positions beyond 32 bits
+        ordered = torch.cat([g.sort().values for g in groups])
     with _lib.on_device(dev):
         _lib.check(lib.omni_lloyd_max_fit(_lib.ptr(ordered), total, _lib.ptr(offsets), len(groups), int(max_iters),
                                           float(tol), _lib.ptr(ws), ws_bytes, _lib.ptr(out), None, _lib.stream_ptr(dev)))
