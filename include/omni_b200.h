@@ -95,6 +95,22 @@ int32_t omni_quantize_heads(const void* x, int32_t dtype, int32_t rotate,
                             const int64_t* out_offsets, int64_t out_offset,
                             void* stream);
 
+/* Smallest and largest of n >= 1 device int64 values into min_max_host[0..1] (page-locked host memory).  Waits for the
+ * stream: a caller that must refuse an append which would run past its cache asks here, once, before it appends. */
+int32_t omni_index_range(const int64_t* values, int64_t n, int64_t* min_max_host, void* stream);
+
+/* One append to a resident cache: T new keys and values per (user, head), quantized (and rotated when rotate != 0) as
+ * omni_quantize_heads would, into rows lens[b] .. lens[b] + T - 1 of the packed arrays [B][H][S][..], the completed groups
+ * of eight V rows converted to the pair layout when pair_v != 0, then lens[b] += T and lens32[b] = lens[b].
+ *   k_strides / v_strides  host int64[3]: element strides of users, heads, tokens (last axis contiguous)
+ *   v_qjl and v_norms may both be NULL (no sign bits and norms for V)
+ *   lens device int64[B] with 0 <= lens[b] <= S - T (the caller has checked: omni_index_range), lens32 device int32[B] */
+int32_t omni_kv_append(const void* k, const void* v, int32_t dtype, int32_t rotate,
+                       const float* codebooks, int32_t cb_per_head, const int32_t* user_ids, int32_t user_id,
+                       int64_t B, int32_t H, int64_t T, const int64_t* k_strides, const int64_t* v_strides,
+                       uint8_t* k_nib, uint8_t* k_qjl, float* k_norms, uint8_t* v_nib, uint8_t* v_qjl, float* v_norms,
+                       int64_t S, int64_t* lens, int32_t* lens32, int32_t pair_v, void* stream);
+
 /* Inverse codec to fp32 out[B][H][T][128] (kernels/quantize.py:593-640 `dequantize_heads`).
  * Packed inputs use row strides is_b, is_h as above; with_qjl == 0 gives cb[code] only. */
 int32_t omni_dequantize_heads(const uint8_t* nib, const uint8_t* qjl, const float* norms,

@@ -27,6 +27,9 @@ SIGNATURES = {
     "omni_rotate": (_i32, [_vp, _vp, _i64, _i32, _vp]),
     "omni_quantize_heads": (_i32, [_vp, _i32, _i32, _vp, _i32, _vp, _i32, _i64, _i32, _i64, _i64, _i64, _i64,
                                    _vp, _vp, _vp, _i64, _i64, _vp, _i64, _vp]),
+    "omni_index_range": (_i32, [_vp, _i64, _vp, _vp]),
+    "omni_kv_append": (_i32, [_vp, _vp, _i32, _i32, _vp, _i32, _vp, _i32, _i64, _i32, _i64, _vp, _vp,
+                              _vp, _vp, _vp, _vp, _vp, _vp, _i64, _vp, _vp, _i32, _vp]),
     "omni_dequantize_heads": (_i32, [_vp, _vp, _vp, _vp, _i32, _vp, _i32, _i64, _i32, _i64, _i64, _i64, _i32,
                                      _vp, _vp]),
     "omni_quantize_rows": (_i32, [_vp, _vp, _i32, _i32, _i64, _vp, _vp, _vp, _vp]),
@@ -151,6 +154,19 @@ def stream_ptr(device: torch.device):
     """Raw handle of torch's current stream on ``device``."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     return torch._C._cuda_getCurrentRawStream(idx) or None
+
+
+def index_range(x: torch.Tensor):
+    """(smallest, largest) of a non-empty integer tensor.  One launch and one wait where the library can read the tensor
+    as it is (``.min()`` and ``.max()`` are two of each)."""
+    if x.is_cuda and x.dtype is torch.int64 and x.is_contiguous() and x.numel() > 0 and not torch.cuda.is_current_stream_capturing():
+        dev = x.device
+        got = torch.empty(2, dtype=torch.int64, pin_memory=True)
+        with on_device(dev):
+            check(ensure_init(dev).omni_index_range(x.data_ptr(), x.numel(), got.data_ptr(), stream_ptr(dev)))
+        lo, hi = got.tolist()
+        return lo, hi
+    return int(x.min()), int(x.max())
 
 
 _workspaces = {}

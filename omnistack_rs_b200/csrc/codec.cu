@@ -278,6 +278,31 @@ static int32_t for_each_seed_block(int32_t base, int32_t user_id, int64_t n_rows
     return OMNI_OK;
 }
 
+// Smallest and largest of n values; one CTA (a cache has at most some ten thousand users).
+__global__ void __launch_bounds__(1024) index_range_kernel(const int64_t* v, int64_t n, int64_t* out) {
+    __shared__ long long lo_s[32], hi_s[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    long long lo = v[0], hi = v[0];
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) { const long long x = v[i]; lo = x < lo ? x : lo; hi = x > hi ? x : hi; }
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) {
+        const long long l = __shfl_xor_sync(kFullMask, lo, m), h = __shfl_xor_sync(kFullMask, hi, m);
+        lo = l < lo ? l : lo; hi = h > hi ? h : hi;
+    }
+    if (lane == 0) { lo_s[warp] = lo; hi_s[warp] = hi; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < (int)blockDim.x / 32; ++k) { lo = lo_s[k] < lo ? lo_s[k] : lo; hi = hi_s[k] > hi ? hi_s[k] : hi; }
+        out[0] = lo; out[1] = hi;
+    }
+}
+
+// After an append: the users' lengths, as the codec's offsets (int64) and as attention takes them (int32).
+__global__ void __launch_bounds__(256) advance_lengths_kernel(int64_t* lens, int32_t* lens32, int64_t n, int64_t by) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) { const int64_t v = lens[i] + by; lens[i] = v; lens32[i] = (int32_t)v; }
+}
+
 static int32_t quantize_common(CodecArgs& a, int32_t dtype, int32_t rotate, void* stream) {
     if (!a.g_rows) {
         const DeviceTables* tb = tables_for_current_device();
@@ -351,6 +376,49 @@ extern "C" int32_t omni_quantize_heads(const void* x, int32_t dtype, int32_t rot
     a.nib = nib; a.qjl = qjl; a.norms = norms; a.os_b = os_b; a.os_h = os_h;
     a.out_offsets = out_offsets; a.out_offset = out_offset;
     return quantize_common(a, dtype, rotate, stream);
+}
+
+extern "C" int32_t omni_index_range(const int64_t* values, int64_t n, int64_t* min_max_host, void* stream) {
+    OMNI_REQUIRE(n >= 1 && values && min_max_host, OMNI_ERR_ARG, "omni_index_range: no values or NULL buffer");
+    void* out = nullptr;
+    OMNI_CUDA(cudaHostGetDevicePointer(&out, min_max_host, 0));
+    index_range_kernel<<<1, n <= 256 ? 128 : 1024, 0, (cudaStream_t)stream>>>(values, n, (int64_t*)out);
+    OMNI_CUDA(cudaGetLastError());
+    return check_cuda(cudaStreamSynchronize((cudaStream_t)stream), "omni_index_range");
+}
+
+extern "C" int32_t omni_kv_append(const void* k, const void* v, int32_t dtype, int32_t rotate,
+                                  const float* codebooks, int32_t cb_per_head, const int32_t* user_ids, int32_t user_id,
+                                  int64_t B, int32_t H, int64_t T, const int64_t* k_strides, const int64_t* v_strides,
+                                  uint8_t* k_nib, uint8_t* k_qjl, float* k_norms, uint8_t* v_nib, uint8_t* v_qjl, float* v_norms,
+                                  int64_t S, int64_t* lens, int32_t* lens32, int32_t pair_v, void* stream) {
+    OMNI_REQUIRE(k_strides && v_strides && lens && lens32, OMNI_ERR_ARG, "omni_kv_append: NULL strides or lengths");
+    OMNI_REQUIRE(B >= 0 && H >= 0 && T >= 0, OMNI_ERR_ARG, "omni_kv_append: negative extent");
+    if (B == 0 || H == 0 || T == 0) return OMNI_OK;
+    const DeviceTables* tb = tables_for_current_device();
+    if (!tb) return OMNI_ERR_NOT_INIT;
+    // keys and values in one launch when the fast kernel covers both and they have the same kind of output
+    const FastQuantArgs f[2] = {{k, k_strides[0], k_strides[1], k_strides[2], codebooks, cb_per_head, user_ids, user_id, B, H, T,
+                                 k_nib, k_qjl, k_norms, (int64_t)H * S, S, lens, 0, tb->rows},
+                                {v, v_strides[0], v_strides[1], v_strides[2], codebooks, cb_per_head, user_ids, user_id, B, H, T,
+                                 v_nib, v_qjl, v_norms, (int64_t)H * S, S, lens, 0, tb->rows}};
+    if (!getenv("OMNI_QUANT_KERNEL") && codebooks && k && v && k_nib && v_nib && (k_qjl != nullptr) == (v_qjl != nullptr) && H <= kSeeds &&
+        fast_quantize_eligible(f[0], dtype) && fast_quantize_eligible(f[1], dtype)) {
+        const int32_t rc = launch_fast_quantize_jobs(f, 2, dtype, rotate, (cudaStream_t)stream);
+        if (rc != OMNI_OK) return rc;
+    } else {
+        for (const FastQuantArgs& j : f) {
+            const int32_t rc = omni_quantize_heads(j.x, dtype, rotate, codebooks, cb_per_head, user_ids, user_id, B, H, T, j.xs_b, j.xs_h, j.xs_t,
+                                                   j.nib, j.qjl, j.norms, j.os_b, j.os_h, lens, 0, stream);
+            if (rc != OMNI_OK) return rc;
+        }
+    }
+    if (pair_v) {
+        const int32_t rc = launch_v_pair_grown(v_nib, B, H, S, lens, T, (cudaStream_t)stream);
+        if (rc != OMNI_OK) return rc;
+    }
+    advance_lengths_kernel<<<(unsigned)((B + 255) / 256), 256, 0, (cudaStream_t)stream>>>(lens, lens32, B, T);
+    return check_cuda(cudaGetLastError(), "advance_lengths_kernel launch");
 }
 
 extern "C" int32_t omni_quantize_rows(const float* x, const float* codebook, int32_t base_head_idx, int32_t user_id,

@@ -336,8 +336,9 @@ __device__ __forceinline__ void stage_row(uint32_t buf, const void* x, int64_t i
 // SIGNS = false: only the nibble rows are produced (a.qjl and a.norms are null): V rows of a cache whose attention
 // never reads their sign bits or norms skip the projections altogether.
 template <int DT, bool ROTATE, bool SIGNS>
-__global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(FastQuantArgs a) {
+__global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(const __grid_constant__ FastQuantJobs jobs) {
     extern __shared__ __align__(256) unsigned char fq_smem[];
+    const FastQuantArgs& a = jobs.job[blockIdx.y];
     const int n_tabs = a.cb_per_head ? a.H : 1;
     HeadTables* tabs = reinterpret_cast<HeadTables*>(fq_smem);
     uint4* gfrag_all = reinterpret_cast<uint4*>(fq_smem + sizeof(HeadTables) * n_tabs);
@@ -715,8 +716,10 @@ bool fast_quantize_eligible(const FastQuantArgs& a, int dtype) {
     return a.T > 0 && a.T <= 0x7ffffff0LL && a.B * a.H * ((a.T + 7) >> 3) < 0xffffffffLL;
 }
 
+// One launch for one call, or for two calls of the same extents (keys and values of one append): grid.y = jobs.
 template <int DT>
-static int32_t launch_fast_t(const FastQuantArgs& a, int rotate, cudaStream_t st) {
+static int32_t launch_fast_t(const FastQuantArgs* jobs, int n_jobs, int rotate, cudaStream_t st) {
+    const FastQuantArgs& a = jobs[0];
     int dev = 0, sms = 148;
     OMNI_CUDA(cudaGetDevice(&dev));
     OMNI_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -724,8 +727,10 @@ static int32_t launch_fast_t(const FastQuantArgs& a, int rotate, cudaStream_t st
     const size_t smem = sizeof(HeadTables) * n_tabs + (size_t)kFqWarps * 16 * 32 * sizeof(uint4) +
                         (size_t)kFqWarps * (kStageBytesPerWarp + kBallotBytesPerWarp);
     const int64_t groups = a.B * a.H * ((a.T + 7) >> 3);
-    // two resident CTAs per SM; fewer groups than warps are spread over the SMs, one group per warp
-    const int64_t blocks = groups < 2 * sms ? groups : 2 * sms;
+    // two resident CTAs per SM, over both jobs while these have no more groups than warps (a second wave would build its
+    // tables after the first one's work: K and V of one token for 64 users x 8 heads 20.6 us against 12.0 us); fewer groups than warps are spread over the SMs, one group per warp
+    const int64_t most = n_jobs * groups <= 2 * sms * kFqWarps ? 2 * sms / n_jobs : 2 * sms;
+    const int64_t blocks = groups < most ? groups : most;
     const bool signs = a.qjl != nullptr;
     auto kern = signs ? (rotate ? fast_quantize_kernel<DT, true, true> : fast_quantize_kernel<DT, false, true>)
                       : (rotate ? fast_quantize_kernel<DT, true, false> : fast_quantize_kernel<DT, false, false>);
@@ -743,7 +748,10 @@ static int32_t launch_fast_t(const FastQuantArgs& a, int rotate, cudaStream_t st
             done.emplace_back(key, dev);
         }
     }
-    kern<<<(unsigned)blocks, kFqWarps * 32, smem, st>>>(a);
+    FastQuantJobs j;
+    j.job[0] = jobs[0];
+    j.job[1] = jobs[n_jobs - 1];
+    kern<<<dim3((unsigned)blocks, (unsigned)n_jobs), kFqWarps * 32, smem, st>>>(j);
     return check_cuda(cudaGetLastError(), "fast_quantize_kernel launch");
 }
 
@@ -769,10 +777,14 @@ int32_t launch_fast_quantize(const FastQuantArgs& a, int dtype, int rotate, cuda
             case OMNI_F16:  return launch_tc_t<OMNI_F16>(a, rotate, st);
         }
     }
+    return launch_fast_quantize_jobs(&a, 1, dtype, rotate, st);
+}
+
+int32_t launch_fast_quantize_jobs(const FastQuantArgs* jobs, int n_jobs, int dtype, int rotate, cudaStream_t st) {
     switch (dtype) {
-        case OMNI_F32:  return launch_fast_t<OMNI_F32>(a, rotate, st);
-        case OMNI_BF16: return launch_fast_t<OMNI_BF16>(a, rotate, st);
-        case OMNI_F16:  return launch_fast_t<OMNI_F16>(a, rotate, st);
+        case OMNI_F32:  return launch_fast_t<OMNI_F32>(jobs, n_jobs, rotate, st);
+        case OMNI_BF16: return launch_fast_t<OMNI_BF16>(jobs, n_jobs, rotate, st);
+        case OMNI_F16:  return launch_fast_t<OMNI_F16>(jobs, n_jobs, rotate, st);
     }
     return set_error(OMNI_ERR_ARG, "unknown dtype code %d", dtype);
 }

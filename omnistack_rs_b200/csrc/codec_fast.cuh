@@ -14,9 +14,15 @@ struct FastQuantArgs {
     const uint32_t* g_rows;
 };
 
+// One or two calls served by one launch: same extents, codebooks, user ids and kind of output (sign bits or not).
+struct FastQuantJobs { FastQuantArgs job[2]; };
+
 // true when the fast kernel covers this call (shape, alignment); the caller falls back otherwise
 bool fast_quantize_eligible(const FastQuantArgs& a, int dtype);
 int32_t launch_fast_quantize(const FastQuantArgs& a, int dtype, int rotate, cudaStream_t st);
+int32_t launch_fast_quantize_jobs(const FastQuantArgs* jobs, int n_jobs, int dtype, int rotate, cudaStream_t st);
+// qattn.cu: the groups of eight V rows completed by appending `grow` keys at each user's length, to the pair layout
+int32_t launch_v_pair_grown(uint8_t* v_nib, int64_t B, int H, int64_t S, const int64_t* lens, int64_t grow, cudaStream_t st);
 
 // stand-alone rotation of n_rows contiguous rows (16-byte aligned buffers)
 int32_t launch_fast_rotate(const void* x, void* y, int64_t n_rows, int dtype, cudaStream_t st);

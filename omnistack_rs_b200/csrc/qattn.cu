@@ -13,6 +13,7 @@
 // exactly as the codec does (kernels/quantize.py:583), which is what the reference's
 // CPU path (kernels/fused_attention.py:435-466) computes.
 #include "qattn.cuh"
+#include "codec_fast.cuh"
 #include "qattn_lane.cuh"
 #include <mutex>
 #include <cstdlib>
@@ -97,7 +98,7 @@ __global__ void __launch_bounds__(kCombineWarps * 32) qattn_combine_kernel(const
 // saves the shift-and-merge per lookup.  Within a group of eight consecutive keys the pairs are (0,3), (1,2), (4,7),
 // (5,6); the row of the pair's first key receives the even-d nibbles of both keys (byte j = code[a][2j] |
 // code[b][2j] << 4), the row of the second key the odd-d nibbles.  The transform is its own inverse.  One warp
-// converts one group: lane = (pair, 8-byte column).
+// converts one group: lane = (pair, 8-byte column).  With lens_before alone, len_after is the number of keys added to each.
 __global__ void __launch_bounds__(256) v_pair_groups_kernel(uint8_t* v_nib, int64_t B, int H, int64_t ks_b, int64_t ks_h,
                                                             const int64_t* lens_before, int64_t len_before,
                                                             const int64_t* lens_after, int64_t len_after, int64_t max_groups) {
@@ -108,7 +109,9 @@ __global__ void __launch_bounds__(256) v_pair_groups_kernel(uint8_t* v_nib, int6
         const int64_t gi = u % max_groups, bh = u / max_groups;
         const int h = (int)(bh % H);
         const int64_t b = bh / H;
-        const int64_t g0 = (lens_before ? lens_before[b] : len_before) >> 3, g1 = (lens_after ? lens_after[b] : len_after) >> 3;
+        const int64_t before = lens_before ? lens_before[b] : len_before;
+        const int64_t after = lens_after ? lens_after[b] : (lens_before ? before + len_after : len_after);
+        const int64_t g0 = before >> 3, g1 = after >> 3;
         const int64_t grp = g0 + gi;                    // groups [g0, g1) became complete with this append
         if (grp >= g1) continue;
         const int pair = lane >> 3, col = lane & 7;
@@ -123,6 +126,15 @@ __global__ void __launch_bounds__(256) v_pair_groups_kernel(uint8_t* v_nib, int6
         *pa = x;
         *pb = y;
     }
+}
+
+int32_t launch_v_pair_grown(uint8_t* v_nib, int64_t B, int H, int64_t S, const int64_t* lens, int64_t grow, cudaStream_t st) {
+    OMNI_REQUIRE(v_nib && (reinterpret_cast<uintptr_t>(v_nib) & 7) == 0, OMNI_ERR_ARG, "omni_kv_append: NULL or misaligned V nibble array");
+    const int64_t max_groups = (grow + 7) / 8;            // groups [len / 8, (len + grow) / 8): at most this many for any len
+    int64_t blocks = (B * H * max_groups + 7) / 8;
+    if (blocks > 148 * 32) blocks = 148 * 32;
+    v_pair_groups_kernel<<<(unsigned)blocks, 256, 0, st>>>(v_nib, B, H, (int64_t)H * S, S, lens, 0, nullptr, grow, max_groups);
+    return check_cuda(cudaGetLastError(), "v_pair_groups_kernel launch");
 }
 
 static bool aligned(const void* p, size_t a) { return (reinterpret_cast<uintptr_t>(p) % a) == 0; }

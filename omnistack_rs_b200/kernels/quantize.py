@@ -48,6 +48,13 @@ def _user_args(user_id: Union[int, torch.Tensor], B: int, dev):
     return None, uid
 
 
+def _codec_rows(x: torch.Tensor) -> torch.Tensor:
+    """``x`` itself when the codec can read its rows in place, else a contiguous copy."""
+    if x.stride(-1) != 1 or any(s % 4 for s in x.stride()[:-1]) or x.data_ptr() % 16:
+        return x.contiguous()
+    return x
+
+
 def _quantize_into(x, codebooks, user_id, rotate, nib, qjl, norms, os_b, os_h, out_offsets, out_offset):
     B, H, T, D = x.shape
     if D != HEAD_DIM:
@@ -56,8 +63,7 @@ def _quantize_into(x, codebooks, user_id, rotate, nib, qjl, norms, os_b, os_h, o
     if x.dtype not in _lib.DTYPE_CODE:
         raise TypeError(f"unsupported dtype {x.dtype}")
     lib = _lib.ensure_init(dev)
-    if x.stride(-1) != 1 or any(s % 4 for s in x.stride()[:-1]) or x.data_ptr() % 16:
-        x = x.contiguous()
+    x = _codec_rows(x)
     cb, per_head = _prep_codebooks(codebooks, H, dev)
     ids, uid = _user_args(user_id, B, dev)
     offs = None
@@ -101,7 +107,8 @@ def rotate_quantize_append(x_new: torch.Tensor, cache_nib: torch.Tensor, cache_q
     if not (cache_nib.is_contiguous() and (cache_qjl is None or (cache_qjl.is_contiguous() and cache_norms.is_contiguous()))):
         raise ValueError("cache tensors must be contiguous")
     if isinstance(offsets, torch.Tensor):
-        if int(offsets.max()) + T > S_max or int(offsets.min()) < 0:
+        lo, hi = _lib.index_range(offsets)
+        if hi + T > S_max or lo < 0:
             raise ValueError("append would run past the cache capacity")
         _quantize_into(x_new, codebooks, user_id, rotate, cache_nib, cache_qjl, cache_norms,
                        H * S_max, S_max, offsets, 0)

@@ -8,6 +8,7 @@ block of users and no collective is needed on the data path.
 """
 from __future__ import annotations
 
+import ctypes as C
 import math
 import os
 from typing import Optional, Tuple
@@ -15,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from .kernels.quantize import _NBYTES_NIBBLE, _NBYTES_QJL, _prep_codebooks, rotate_quantize_append
+from .kernels.quantize import _NBYTES_NIBBLE, _NBYTES_QJL, _codec_rows, _prep_codebooks, _user_args, rotate_quantize_append
 from .kernels.fused_attention import _qattn, _auto_splits, pair_v_rows
 
 HEAD_DIM = 128
@@ -149,6 +150,8 @@ class QuantizedKVCache:
         """Quantize-append ``(n_users, n_kv_heads, T_new, 128)`` keys and values for every
         user at its current length."""
         T = k_new.shape[2]
+        if self._append_together(k_new, v_new, T, rotate):
+            return
         if int(self.lens.max()) + T > self.max_len:
             raise ValueError("append would run past the cache capacity")
         rotate_quantize_append(k_new, self.k_nib, self.k_qjl, self.k_norms, self.lens, self.codebooks,
@@ -159,6 +162,43 @@ class QuantizedKVCache:
             pair_v_rows(self.v_nib, self.lens, self.lens + T)
         self.lens += T
         self.lens32.copy_(self.lens)
+
+    def _append_together(self, k_new, v_new, T: int, rotate: bool) -> bool:
+        """The whole append as one library call behind one check of the lengths (``omni_kv_append``: both codec passes in
+        one launch, the pair layout and the new lengths after them), for keys and values of one shape and dtype and the
+        cache's own tensors as the constructor made them.  False: nothing was done, the general path takes the call.
+        (Separate calls wait for the device five times to check the lengths and launch six kernels: one token for 64
+        users, appended and attended to, 233 us against 96 us.)"""
+        n, H, S, _ = self.k_nib.shape
+        dev = self.k_nib.device
+        packed = [(self.k_nib, _NBYTES_NIBBLE), (self.k_qjl, _NBYTES_QJL), (self.v_nib, _NBYTES_NIBBLE), (self.v_qjl, _NBYTES_QJL)]
+        norms = [self.k_norms, self.v_norms]
+        if not (dev.type == "cuda" and T > 0 and n > 0 and k_new.shape == v_new.shape == (n, H, T, HEAD_DIM)
+                and k_new.dtype == v_new.dtype and k_new.dtype in _lib.DTYPE_CODE and k_new.device == v_new.device == dev
+                and S == self.max_len and self.k_qjl is not None and self.k_norms is not None
+                and (self.v_qjl is None) == (self.v_norms is None)
+                and all(t is None or (t.shape == (n, H, S, w) and t.dtype is torch.uint8) for t, w in packed)
+                and all(t is None or (t.shape == (n, H, S) and t.dtype is torch.float32) for t in norms)
+                and self.lens.shape == self.lens32.shape == (n,) and self.lens.dtype is torch.int64 and self.lens32.dtype is torch.int32
+                and all(t is None or (t.device == dev and t.is_contiguous())
+                        for t in [t for t, _ in packed] + norms + [self.lens, self.lens32])
+                and not torch.cuda.is_current_stream_capturing()):
+            return False
+        lo, hi = _lib.index_range(self.lens)
+        if hi + T > self.max_len or lo < 0:
+            raise ValueError("append would run past the cache capacity")
+        lib = _lib.ensure_init(dev)
+        k_new, v_new = _codec_rows(k_new), _codec_rows(v_new)
+        cb, per_head = _prep_codebooks(self.codebooks, H, dev)
+        ids, uid = _user_args(self.user_ids, n, dev)
+        strides = [(C.c_int64 * 3)(*t.stride()[:3]) for t in (k_new, v_new)]
+        with _lib.on_device(dev):
+            _lib.check(lib.omni_kv_append(
+                _lib.ptr(k_new), _lib.ptr(v_new), _lib.DTYPE_CODE[k_new.dtype], int(bool(rotate)), _lib.ptr(cb), per_head,
+                _lib.ptr(ids), uid, n, H, T, strides[0], strides[1],
+                _lib.ptr(self.k_nib), _lib.ptr(self.k_qjl), _lib.ptr(self.k_norms), _lib.ptr(self.v_nib), _lib.ptr(self.v_qjl),
+                _lib.ptr(self.v_norms), S, _lib.ptr(self.lens), _lib.ptr(self.lens32), int(self.pair_v), _lib.stream_ptr(dev)))
+        return True
 
     def attend(self, q: torch.Tensor, scale: Optional[float] = None, with_qjl: bool = True,
                rotate_q: bool = False, unrotate_out: bool = False, n_splits: Optional[int] = None) -> torch.Tensor:
