@@ -262,6 +262,21 @@ int32_t omni_qattn_decode_lora(const void* q, int32_t q_dtype,
                                int32_t n_splits, void* workspace, size_t workspace_bytes,
                                float* out, int32_t* status_word, void* stream, const omni_lora_t* lora);
 
+/* What stays the same between the decode calls of a serving loop: every argument of omni_qattn_decode_lora but the query,
+ * the output, the workspace, the adapters and the stream.  A host fills it once; omni_qattn_decode_call then marshals seven
+ * arguments per call instead of thirty-one. */
+typedef struct omni_qattn_call_t {
+    const uint8_t* k_nib; const uint8_t* k_qjl; const float* k_norms; const uint8_t* v_nib;
+    const float* codebooks; const int32_t* user_ids; const int32_t* seq_lens; const int32_t* cache_slots;
+    int32_t* status_word;
+    int64_t B, S, ks_b, ks_h;
+    int32_t q_dtype, cb_per_head, user_id, Hq, Hkv, T;
+    int32_t with_qjl, rotate_q, unrotate_out, v_paired, n_splits;
+    float   scale;
+} omni_qattn_call_t;
+int32_t omni_qattn_decode_call(const omni_qattn_call_t* call, const void* q, float* out, void* workspace, size_t workspace_bytes,
+                               const omni_lora_t* lora, void* stream);
+
 /* Allocation-free decode attention.  No counterpart in the reference: it exists for hosts
  * that must not allocate device memory when they call into this library -- an inference
  * server or plugin host that owns the whole device heap and hands its plugins fixed

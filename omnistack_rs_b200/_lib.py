@@ -44,6 +44,7 @@ SIGNATURES = {
     "omni_qattn_decode_lora": (_i32, [_vp, _i32, _vp, _vp, _vp, _vp, _vp, _i32, _vp, _i32, _vp, _vp,
                                       _i64, _i32, _i32, _i32, _i64, _i64, _i64, _f32, _i32, _i32, _i32, _i32, _i32,
                                       _vp, _sz, _vp, _vp, _vp, _vp]),
+    "omni_qattn_decode_call": (_i32, [_vp, _vp, _vp, _vp, _sz, _vp, _vp]),
     "omni_qjl_encode_bool": (_i32, [_vp, _i64, _i32, _vp, _vp, _vp]),
     "omni_qjl_reconstruct_bool": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp]),
     "omni_lloyd_max_workspace_bytes": (_sz, [_i64]),
@@ -135,12 +136,21 @@ class OmniLora(C.Structure):
                 ("n_adapters", C.c_int32), ("hidden", C.c_int32), ("rank", C.c_int32), ("alpha", C.c_float)]
 
 
+class OmniCall(C.Structure):
+    """``omni_qattn_call_t`` of the C header."""
+    _fields_ = ([(n, C.c_void_p) for n in ("k_nib", "k_qjl", "k_norms", "v_nib", "codebooks", "user_ids", "seq_lens", "cache_slots", "status_word")]
+                + [(n, C.c_int64) for n in ("B", "S", "ks_b", "ks_h")]
+                + [(n, C.c_int32) for n in ("q_dtype", "cb_per_head", "user_id", "Hq", "Hkv", "T", "with_qjl", "rotate_q", "unrotate_out",
+                                            "v_paired", "n_splits")]
+                + [("scale", C.c_float)])
+
+
 _NULL_CONTEXT = contextlib.nullcontext()
 
 
 def on_device(device: torch.device):
     """Context manager that makes ``device`` current (free when it already is)."""
-    if device.index is None or torch.cuda.current_device() == device.index:
+    if device.index is None or torch._C._cuda_getDevice() == device.index:
         return _NULL_CONTEXT
     return torch.cuda.device(device)
 

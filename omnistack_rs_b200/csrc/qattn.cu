@@ -411,6 +411,15 @@ extern "C" int32_t omni_qattn_decode_lora(const void* q, int32_t q_dtype,
     return launch(a, (cudaStream_t)stream, workspace_bytes - (B == 0 || T == 0 ? 0 : qb));
 }
 
+extern "C" int32_t omni_qattn_decode_call(const omni_qattn_call_t* c, const void* q, float* out, void* workspace, size_t workspace_bytes,
+                                          const omni_lora_t* lora, void* stream) {
+    OMNI_REQUIRE(c != nullptr, OMNI_ERR_ARG, "omni_qattn_decode_call: call is NULL");
+    return omni_qattn_decode_lora(q, c->q_dtype, c->k_nib, c->k_qjl, c->k_norms, c->v_nib, c->codebooks, c->cb_per_head, c->user_ids, c->user_id,
+                                  c->seq_lens, c->cache_slots, c->B, c->Hq, c->Hkv, c->T, c->S, c->ks_b, c->ks_h, c->scale, c->with_qjl,
+                                  c->rotate_q, c->unrotate_out, c->v_paired, c->n_splits, workspace, workspace_bytes, out, c->status_word,
+                                  stream, lora);
+}
+
 extern "C" int32_t omni_qattn_decode_host(const void* q_host, int32_t q_dtype, void* q_stage,
                                           const uint8_t* k_nib, const uint8_t* k_qjl, const float* k_norms,
                                           const uint8_t* v_nib, const float* codebooks, int32_t cb_per_head,
