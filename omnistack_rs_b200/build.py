@@ -17,7 +17,7 @@ import sys
 CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "csrc")
 OBJ_DIR = os.path.join(CSRC, "_obj")
 LIB_PATH = os.path.join(CSRC, "libomni_b200.so")
-SOURCES = ["runtime.cu", "codec.cu", "codec_fast.cu", "qattn.cu", "qattn_mma.cu", "qattn_mma_lora.cu", "qattn_umma.cu", "lora_q.cu",
+SOURCES = ["runtime.cu", "codec.cu", "codec_fast.cu", "qattn.cu", "qattn_mma.cu", "qattn_mma_lora.cu", "qattn_umma.cu", "qattn_short.cu", "lora_q.cu",
            "lloyd_max.cu", "qjl_bool.cu"]
 # qattn_mma.cu is also a header: qattn_mma_lora.cu includes it
 HEADERS = ["common.cuh", "qattn.cuh", "qattn_lane.cuh", "codec_fast.cuh", "codec_tc.cuh", "qattn_mma.cu", os.path.join("..", "..", "include", "omni_b200.h")]

@@ -196,15 +196,16 @@ static int32_t validate(const AttnArgs& a, size_t ws_bytes) {
     return OMNI_OK;
 }
 
-enum KernelChoice { kAuto = 0, kLanePerKey = 1, kMma = 2, kUmma = 3 };
+enum KernelChoice { kAuto = 0, kLanePerKey = 1, kMma = 2, kUmma = 3, kShort = 4 };
 
-// OMNI_QATTN_KERNEL=lane|mma|umma forces one kernel where it covers the call (tests and profiling); default: by shape.
+// OMNI_QATTN_KERNEL=lane|mma|umma|short forces one kernel where it covers the call (tests and profiling); default: by shape.
 static KernelChoice kernel_choice_from_env() {
     const char* e = getenv("OMNI_QATTN_KERNEL");
     if (!e) return kAuto;
     if (e[0] == 'l') return kLanePerKey;
     if (e[0] == 'm') return kMma;
     if (e[0] == 'u') return kUmma;
+    if (e[0] == 's') return kShort;
     return kAuto;
 }
 
@@ -213,21 +214,21 @@ static KernelChoice kernel_choice_from_env() {
 // 56 columns = seven tiles 0.247 vs 0.303 ms, 128 columns 0.259 vs 0.546 ms).
 constexpr int64_t kUmmaMinColumns = 49;
 
-// Which tensor-core kernel serves a call, if any (otherwise the lane-per-key kernel does).
-// Measured crossover: the warp-level kernel wins from 128 keys on, and for shorter caches once the lane-per-key
-// kernel would need more than about a thousand warps.
-static void choose_kernels(const AttnArgs& a, bool* use_umma, bool* use_mma) {
+// Which kernel serves a call; kLanePerKey when none of the others does.
+static KernelChoice choose_kernel(const AttnArgs& a) {
     const KernelChoice choice = kernel_choice_from_env();
     const int64_t cols = (int64_t)(a.Hq / a.Hkv) * a.T;
-    *use_umma = umma_eligible(a) && (choice == kUmma || (choice == kAuto && cols >= kUmmaMinColumns && a.S >= 128));
-    *use_mma = !*use_umma && mma_eligible(a) &&
-               (choice == kMma || ((choice == kAuto || choice == kUmma) && (a.S >= 128 || a.B * a.Hq * a.T >= 1024)));
+    if (umma_eligible(a) && (choice == kUmma || (choice == kAuto && cols >= kUmmaMinColumns && a.S >= 128))) return kUmma;
+    if (short_eligible(a) && (choice == kShort || (choice == kAuto && short_preferred(a)))) return kShort;
+    if (mma_eligible(a) && (choice == kMma || (choice != kLanePerKey && (a.S >= 128 || a.B * a.Hq * a.T >= 1024)))) return kMma;
+    return kLanePerKey;
 }
 
 static int32_t launch(const AttnArgs& a, cudaStream_t st, size_t ws_bytes) {
     if (a.B == 0 || a.T == 0) return OMNI_OK;
-    bool use_umma, use_mma;
-    choose_kernels(a, &use_umma, &use_mma);
+    const KernelChoice kernel = choose_kernel(a);
+    if (kernel == kShort) return launch_short(a, st);
+    const bool use_umma = kernel == kUmma, use_mma = kernel == kMma;
     OMNI_REQUIRE(!(use_umma && a.lora.x), OMNI_ERR_UNSUPPORTED, "qattn: the tcgen05 kernel takes no folded query update");
     if (use_umma) {
         const int32_t rc = launch_umma(a, st);
@@ -424,11 +425,10 @@ extern "C" int32_t omni_qattn_decode_lora(const void* q, int32_t q_dtype,
     // benchmark's shape, rank 16 / hidden 128), the separate launch otherwise.  OMNI_LORA_FOLD=1 folds wherever the
     // serving kernel can, OMNI_LORA_FOLD=0 never.
     const char* fold_env = getenv("OMNI_LORA_FOLD");
-    bool use_umma = false, use_mma = false;
-    if (B > 0 && T > 0) choose_kernels(a, &use_umma, &use_mma);
-    const bool fold = (fold_env && fold_env[0] == '1') ? !use_umma
+    const KernelChoice kernel = B > 0 && T > 0 ? choose_kernel(a) : kLanePerKey;
+    const bool fold = (fold_env && fold_env[0] == '1') ? kernel != kUmma
                     : (fold_env && fold_env[0] == '0') ? false
-                    : (use_mma && lora->rank <= 32 && (int64_t)lora->rank * lora->hidden <= 8192);
+                    : ((kernel == kMma || kernel == kShort) && lora->rank <= 32 && (int64_t)lora->rank * lora->hidden <= 8192);
     if (fold && B > 0 && T > 0) {
         OMNI_REQUIRE(lora->hidden > 0 && lora->rank > 0 && lora->n_adapters >= 0, OMNI_ERR_ARG, "qattn_decode_lora: bad extent");
         OMNI_REQUIRE(lora->rank <= kLoraFoldMaxRank, OMNI_ERR_UNSUPPORTED, "qattn_decode_lora: rank %d exceeds %d", lora->rank, kLoraFoldMaxRank);

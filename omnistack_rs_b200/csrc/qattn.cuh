@@ -286,6 +286,10 @@ static __device__ __noinline__ bool lora_fold_tile(const LoraFold L, int64_t b, 
 bool mma_eligible(const AttnArgs& a);
 int32_t launch_mma(const AttnArgs& a, cudaStream_t st);
 int32_t launch_mma_lora(const AttnArgs& a, cudaStream_t st);   // qattn_mma_lora.cu: the same kernels with a.lora applied
+// fp32 kernel for short caches (qattn_short.cu): what it can serve, and what it serves best
+bool short_eligible(const AttnArgs& a);
+bool short_preferred(const AttnArgs& a);
+int32_t launch_short(const AttnArgs& a, cudaStream_t st);
 // tcgen05 kernel (qattn_umma.cu): kv heads with many query columns.
 bool umma_eligible(const AttnArgs& a);
 int32_t launch_umma(const AttnArgs& a, cudaStream_t st);
