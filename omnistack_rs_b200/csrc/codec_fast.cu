@@ -335,10 +335,11 @@ __device__ __forceinline__ void stage_row(uint32_t buf, const void* x, int64_t i
 
 // SIGNS = false: only the nibble rows are produced (a.qjl and a.norms are null): V rows of a cache whose attention
 // never reads their sign bits or norms skip the projections altogether.
-template <int DT, bool ROTATE, bool SIGNS>
+// TWO = false: one job, whose arguments are constants of the launch (indexed by block they cost a large call 1 %).
+template <int DT, bool ROTATE, bool SIGNS, bool TWO>
 __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(const __grid_constant__ FastQuantJobs jobs) {
     extern __shared__ __align__(256) unsigned char fq_smem[];
-    const FastQuantArgs& a = jobs.job[blockIdx.y];
+    const FastQuantArgs& a = jobs.job[TWO ? blockIdx.y : 0];
     const int n_tabs = a.cb_per_head ? a.H : 1;
     HeadTables* tabs = reinterpret_cast<HeadTables*>(fq_smem);
     uint4* gfrag_all = reinterpret_cast<uint4*>(fq_smem + sizeof(HeadTables) * n_tabs);
@@ -717,7 +718,7 @@ bool fast_quantize_eligible(const FastQuantArgs& a, int dtype) {
 }
 
 // One launch for one call, or for two calls of the same extents (keys and values of one append): grid.y = jobs.
-template <int DT>
+template <int DT, bool TWO>
 static int32_t launch_fast_t(const FastQuantArgs* jobs, int n_jobs, int rotate, cudaStream_t st) {
     const FastQuantArgs& a = jobs[0];
     int dev = 0, sms = 148;
@@ -732,8 +733,8 @@ static int32_t launch_fast_t(const FastQuantArgs* jobs, int n_jobs, int rotate, 
     const int64_t most = n_jobs * groups <= 2 * sms * kFqWarps ? 2 * sms / n_jobs : 2 * sms;
     const int64_t blocks = groups < most ? groups : most;
     const bool signs = a.qjl != nullptr;
-    auto kern = signs ? (rotate ? fast_quantize_kernel<DT, true, true> : fast_quantize_kernel<DT, false, true>)
-                      : (rotate ? fast_quantize_kernel<DT, true, false> : fast_quantize_kernel<DT, false, false>);
+    auto kern = signs ? (rotate ? fast_quantize_kernel<DT, true, true, TWO> : fast_quantize_kernel<DT, false, true, TWO>)
+                      : (rotate ? fast_quantize_kernel<DT, true, false, TWO> : fast_quantize_kernel<DT, false, false, TWO>);
     {   // opt in once per (kernel, device) to the shared memory of the largest table count the kernel accepts
         static std::mutex mu;
         static std::vector<std::pair<const void*, int>> done;
@@ -782,9 +783,9 @@ int32_t launch_fast_quantize(const FastQuantArgs& a, int dtype, int rotate, cuda
 
 int32_t launch_fast_quantize_jobs(const FastQuantArgs* jobs, int n_jobs, int dtype, int rotate, cudaStream_t st) {
     switch (dtype) {
-        case OMNI_F32:  return launch_fast_t<OMNI_F32>(jobs, n_jobs, rotate, st);
-        case OMNI_BF16: return launch_fast_t<OMNI_BF16>(jobs, n_jobs, rotate, st);
-        case OMNI_F16:  return launch_fast_t<OMNI_F16>(jobs, n_jobs, rotate, st);
+        case OMNI_F32:  return n_jobs == 2 ? launch_fast_t<OMNI_F32, true>(jobs, 2, rotate, st) : launch_fast_t<OMNI_F32, false>(jobs, 1, rotate, st);
+        case OMNI_BF16: return n_jobs == 2 ? launch_fast_t<OMNI_BF16, true>(jobs, 2, rotate, st) : launch_fast_t<OMNI_BF16, false>(jobs, 1, rotate, st);
+        case OMNI_F16:  return n_jobs == 2 ? launch_fast_t<OMNI_F16, true>(jobs, 2, rotate, st) : launch_fast_t<OMNI_F16, false>(jobs, 1, rotate, st);
     }
     return set_error(OMNI_ERR_ARG, "unknown dtype code %d", dtype);
 }
