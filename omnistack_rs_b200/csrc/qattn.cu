@@ -1,17 +1,6 @@
-// Fused attention over the packed INT4 + QJL cache: the general CUDA-core kernel (small calls and the calls that
-// fold the rotation into q / out), the split-K merge, kernel selection and the C entry points.  The tensor-core
-// kernel that serves every larger call is in qattn_mma.cu.
-//
-// Work unit: one warp per (user, query head, query token, key split).  Lane l walks
-// keys l, l+32, ... of its split with a private online-softmax state (max, sum, 128
-// accumulators); nothing crosses lanes until the final merge.  K and V are dequantised
-// in registers by a 16-entry codebook lookup in shared memory (16 words occupy 16
-// distinct banks, so any access pattern is conflict-free).  The QJL part of K is
-// applied as a score correction  norm * c * sum_i s_i (q . g_i)  with the 64 values
-// (q . g_i) computed once per work unit -- the same algebra as the reference kernel
-// (kernels/fused_attention.py:198-213, 260-276) but with G seeded per (user, kv head)
-// exactly as the codec does (kernels/quantize.py:583), which is what the reference's
-// CPU path (kernels/fused_attention.py:435-466) computes.
+// Fused attention over the packed INT4 + QJL cache: the lane-per-key kernel's launch (its code is in qattn_lane.cuh), the
+// split-K merges, kernel selection and the C entry points.  Short caches are served by qattn_short.cu, larger calls by the
+// tensor-core kernels in qattn_mma.cu and qattn_umma.cu.
 #include "qattn.cuh"
 #include "codec_fast.cuh"
 #include "qattn_lane.cuh"
@@ -260,7 +249,7 @@ static int32_t launch(const AttnArgs& a, cudaStream_t st, size_t ws_bytes) {
         if (rc != OMNI_OK) return rc;
     }
     if (!use_mma) {
-        // The lane-per-key kernel: the call's only kernel for small shapes; behind the tcgen05 kernel it is a
+        // The lane-per-key kernel: the call's only kernel where no other covers it; behind the tcgen05 kernel it is a
         // stand-by that returns at once unless the codebooks are outside the fp16 table's range (decided on the
         // device by both kernels with the same test), so a persistent-size grid suffices there.  (The warp-level kernel
         // runs the same fp32 code itself in that case; a stand-by behind it cost a launch on every call: 64 users x 32 / 8 heads x

@@ -1,5 +1,16 @@
 // The fp32 lane-per-key attention of one warp: the lane-per-key kernel (qattn.cu) and, for codebooks that the fp16 tables
 // cannot hold, the warp-level tensor-core kernel (qattn_mma.cu) run it over their share of the work units.
+//
+// Work unit: one warp per (user, query head, query token, key split).  Lane l walks
+// keys l, l+32, ... of its split with a private online-softmax state (max, sum, 128
+// accumulators); nothing crosses lanes until the final merge.  K and V are dequantised
+// in registers by a 16-entry codebook lookup in shared memory (16 words occupy 16
+// distinct banks, so any access pattern is conflict-free).  The QJL part of K is
+// applied as a score correction  norm * c * sum_i s_i (q . g_i)  with the 64 values
+// (q . g_i) computed once per work unit -- the same algebra as the reference kernel
+// (kernels/fused_attention.py:198-213, 260-276) but with G seeded per (user, kv head)
+// exactly as the codec does (kernels/quantize.py:583), which is what the reference's
+// CPU path (kernels/fused_attention.py:435-466) computes.
 #pragma once
 #include "qattn.cuh"
 

@@ -103,7 +103,7 @@ def _auto_splits(B: int, Hq: int, Hkv: int, T: int, S: int, ragged: bool = False
     orders the users by length), so that the ticket scheduling can even the lengths out, unless every warp has many
     units anyway."""
     if S < 128 and B * Hq * T < 1024:
-        return 1                                   # the lane-per-key kernel's shapes
+        return 1                                   # the short-cache kernel's shapes
     units = max(1, B * Hkv * -(-((Hq // Hkv) * T) // 8))
     rows = B * Hq * T
     best, best_cost, unsplit_cost = 1, float("inf"), float("inf")
