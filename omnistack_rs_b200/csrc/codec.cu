@@ -172,12 +172,18 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) dequantize_kernel(CodecAr
 // the head's 16 centroids (one per lane, fetched by shuffle) and this lane's four columns of G stay in registers
 // for the whole run; per token it reads 2 bytes of codes per lane plus the broadcast sign word and norm, and
 // writes 16 bytes per lane.  kDeqFlight tokens are in flight per iteration.
-constexpr int kDeqRun = 64;     // tokens per work unit
+// Tokens per work unit.  Runs of 64 keep the write streams of a large call long (1,048,576 rows with the sign term: 120.5 us,
+// 121.9 with runs of 16); with fewer than two waves of them, or without the sign term, shorter runs fill the SMs better (320 pairs x
+// 333 rows 22.6 against 18.3 us, 2,000 x 300 79.0 against 73.9, 1,048,576 rows of codes alone 103.3 against 98.0).  The run is a
+// constant of the kernel: as an argument it cost the large call 2 %.
+constexpr int kDeqLongRun = 64, kDeqShortRun = 16;
+constexpr int64_t kDeqLongRunUnits = 12000;
 constexpr int kDeqFlight = 4;   // tokens whose loads are issued together
 
+template <int RUN>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) dequantize_heads_kernel(CodecArgs a) {
     const int lane = threadIdx.x & 31;
-    const int64_t runs_per_head = (a.T + kDeqRun - 1) / kDeqRun;
+    const int64_t runs_per_head = (a.T + RUN - 1) / RUN;
     const int64_t n_units = a.B * a.H * runs_per_head;
     const int64_t nw = (int64_t)gridDim.x * kWarpsPerBlock;
     for (int64_t u = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5); u < n_units; u += nw) {
@@ -192,7 +198,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) dequantize_heads_kernel(C
 #pragma unroll
             for (int k = 0; k < 4; ++k) gc[k] = __ldg(gp + k);
         }
-        const int64_t t_begin = run * kDeqRun, t_end = (t_begin + kDeqRun < a.T) ? t_begin + kDeqRun : a.T;
+        const int64_t t_begin = run * RUN, t_end = (t_begin + RUN < a.T) ? t_begin + RUN : a.T;
         const int64_t in0 = b * a.os_b + h * a.os_h, out0 = (b * a.H + h) * a.T;
         for (int64_t t = t_begin; t < t_end; t += kDeqFlight) {
             uint32_t p[kDeqFlight];
@@ -449,8 +455,12 @@ static int32_t dequantize_common(CodecArgs& a, void* stream) {
         a.g_rows = tb->rows; a.g_cols = tb->cols;
     }
     if (!a.row_seeded) {
-        const int grid = grid_for_rows(a.B * a.H * ((a.T + kDeqRun - 1) / kDeqRun));
-        dequantize_heads_kernel<<<grid, kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(a);
+        const int64_t long_runs = a.B * a.H * ((a.T + kDeqLongRun - 1) / kDeqLongRun);
+        if (a.with_qjl && long_runs >= kDeqLongRunUnits)
+            dequantize_heads_kernel<kDeqLongRun><<<grid_for_rows(long_runs), kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(a);
+        else
+            dequantize_heads_kernel<kDeqShortRun><<<grid_for_rows(a.B * a.H * ((a.T + kDeqShortRun - 1) / kDeqShortRun)), kWarpsPerBlock * 32, 0,
+                                                    (cudaStream_t)stream>>>(a);
         return check_cuda(cudaGetLastError(), "dequantize_heads_kernel launch");
     }
     const int grid = grid_for_rows(a.B * a.H * a.T);
