@@ -172,12 +172,18 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) dequantize_kernel(CodecAr
 // the head's 16 centroids (one per lane, fetched by shuffle) and this lane's four columns of G stay in registers
 // for the whole run; per token it reads 2 bytes of codes per lane plus the broadcast sign word and norm, and
 // writes 16 bytes per lane.  kDeqFlight tokens are in flight per iteration.
-// Tokens per work unit.  Runs of 64 keep the write streams of a large call long (1,048,576 rows with the sign term: 120.5 us,
-// 121.9 with runs of 16); with fewer than two waves of them, or without the sign term, shorter runs fill the SMs better (320 pairs x
-// 333 rows 22.6 against 18.3 us, 2,000 x 300 79.0 against 73.9, 1,048,576 rows of codes alone 103.3 against 98.0).  The run is a
-// constant of the kernel: as an argument it cost the large call 2 %.
+// Tokens per work unit, a constant of the kernel (as an argument it cost the large call 2 %).  Runs of 16 fill the SMs better:
+// 80,000 rows of 64 tokens 12.3 us against 18.7 with runs of 64, 200,000 rows of 70 tokens 29.0 against 43.5; without the sign
+// term also at any size (1,000,000 rows of 1,000 tokens 91.7 against 98.3).  Runs of 64 are taken
+//  - where a pair's tokens fit one of them but leave much of the last run of 16 empty, once the runs of 16 are well more than the
+//    warps that are resident (200,000 rows of 17 tokens 30.3 us against 34.7, of 24 tokens 27.3 against 29.2, of 28 tokens 28.4
+//    against 28.1; 80,000 rows of 20 tokens 11.9 against 12.5, without the sign term 9.6 against 8.9, of 33 tokens 15.4 against
+//    14.4);
+//  - for large calls with the sign term, to which the run makes no difference (1,000,000 rows of 128 tokens 114.9 against 113.8 us;
+//    a case of 1,048,576 rows 120.5 against 121.9).
 constexpr int kDeqLongRun = 64, kDeqShortRun = 16;
 constexpr int64_t kDeqLongRunUnits = 12000;
+constexpr int64_t kDeqResidentWarps = 148 * 32;     // 64 registers a thread
 constexpr int kDeqFlight = 4;   // tokens whose loads are issued together
 
 template <int RUN>
@@ -456,11 +462,14 @@ static int32_t dequantize_common(CodecArgs& a, void* stream) {
     }
     if (!a.row_seeded) {
         const int64_t long_runs = a.B * a.H * ((a.T + kDeqLongRun - 1) / kDeqLongRun);
-        if (a.with_qjl && long_runs >= kDeqLongRunUnits)
+        const int64_t short_runs = a.B * a.H * ((a.T + kDeqShortRun - 1) / kDeqShortRun);
+        const int64_t empty = (kDeqShortRun - a.T % kDeqShortRun) % kDeqShortRun;         // of a pair's last run of 16
+        const bool ragged = a.T <= kDeqLongRun && 4 * empty > a.T;
+        const int64_t resident = kDeqResidentWarps * (a.T > 2 * kDeqShortRun || !a.with_qjl ? 2 : 1);
+        if ((ragged && short_runs > resident) || (a.with_qjl && long_runs >= kDeqLongRunUnits))
             dequantize_heads_kernel<kDeqLongRun><<<grid_for_rows(long_runs), kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(a);
         else
-            dequantize_heads_kernel<kDeqShortRun><<<grid_for_rows(a.B * a.H * ((a.T + kDeqShortRun - 1) / kDeqShortRun)), kWarpsPerBlock * 32, 0,
-                                                    (cudaStream_t)stream>>>(a);
+            dequantize_heads_kernel<kDeqShortRun><<<grid_for_rows(short_runs), kWarpsPerBlock * 32, 0, (cudaStream_t)stream>>>(a);
         return check_cuda(cudaGetLastError(), "dequantize_heads_kernel launch");
     }
     const int grid = grid_for_rows(a.B * a.H * a.T);
