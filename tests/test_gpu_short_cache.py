@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import oracle as orc
+from tests.helpers import device_us
 from tests.test_gpu_attention import make_cache, to_dev, attn_mod
 
 pytestmark = pytest.mark.gpu
@@ -63,7 +64,9 @@ def test_short_cache_rotation_and_slots(dev):
     assert (got - want).abs().max() <= ATOL
 
 
-@pytest.mark.parametrize("Hq,Hkv,T,hid,rank", [(8, 8, 1, 128, 16), (8, 2, 1, 128, 32), (6, 2, 1, 100, 6), (4, 2, 3, 256, 40)])
+@pytest.mark.parametrize("Hq,Hkv,T,hid,rank", [(8, 8, 1, 128, 16), (8, 2, 1, 128, 32), (6, 2, 1, 100, 6), (4, 2, 3, 256, 40),
+                                                (8, 8, 1, 128, 32), (4, 2, 1, 128, 32), (5, 1, 1, 128, 32),       # 1, 2 and 5 columns
+                                                (8, 8, 1, 128, 8), (4, 2, 1, 128, 8), (5, 1, 1, 128, 8)])
 def test_short_cache_query_update(dev, Hq, Hkv, T, hid, rank, monkeypatch):
     """The per-user query update inside the kernel equals the separate launch bit for bit, index -1 leaves the query alone
     and an index past the adapters is reported."""
@@ -90,3 +93,18 @@ def test_short_cache_query_update(dev, Hq, Hkv, T, hid, rank, monkeypatch):
         bad = fa.omni_attn(q.to(dev), *cache, user_id=6, n_splits=1, **lora)
         _lib.check_device_status(dev)
     assert torch.equal(bad, fa.omni_attn(q.to(dev), *cache, user_id=6, n_splits=1))
+
+
+def test_rank_32_costs_little_more_than_rank_16(dev, monkeypatch):
+    """All rows of a rank-32 update are requested ahead, as those of rank 16 (16 users x 8 heads x 50 keys: 5.5 us;
+    with the general form 9.8)."""
+    monkeypatch.delenv("OMNI_QATTN_KERNEL")
+    fa = attn_mod()
+    kn, kq, kr, vn, cb, gen = make_cache(16, 8, 50, seed=1, user_id=3)
+    cache = to_dev(dev, torch.randn(16, 8, 1, 128, generator=gen).to(torch.bfloat16), kn, kq, kr, vn, cb)
+    us = {}
+    for rank in (16, 32):
+        lora = dict(x=torch.randn(16, 1, 128, generator=gen).to(dev), lora_a=torch.randn(4, rank, 128, generator=gen).to(dev),
+                    lora_b=torch.randn(4, 8 * 128, rank, generator=gen).to(dev), lora_indices=(torch.arange(16) % 4).int().to(dev))
+        us[rank] = device_us(lambda: fa.omni_attn(*cache, user_id=3, n_splits=1, **lora))
+    assert us[32] <= 1.35 * us[16], us
