@@ -136,11 +136,14 @@ __device__ __forceinline__ void lora_update(const AttnArgs& a, int64_t b, int hk
 // Builds of the kernel.  The query update's registers set its occupancy (128 of them, four CTAs per SM), so
 //   kAnyUpdate  serves calls without an update and with any;
 //   kRank32     the update of rank 32 with all rows requested ahead, whose registers the others would pay for (16 users x 8 heads x
-//               50 keys 5.5 us against 9.8 with the general form, 128 x 8 x 50 16.0 against 21.3).
-enum ShortBuild { kAnyUpdate, kRank32 };
+//               50 keys 5.5 us against 9.8 with the general form, 128 x 8 x 50 16.0 against 21.3);
+//   kNoUpdate   eight CTAs per SM, for one column and more CTAs than four per SM hold: 127 users x 8 heads x 17 keys 8.2 us against
+//               9.5 (the lane-per-key kernel 9.2); with fewer CTAs its 64 registers are too few (8 CTAs x 256 keys 7.6 against 6.4).
+enum ShortBuild { kAnyUpdate, kRank32, kNoUpdate };
+constexpr int64_t kFourPerSm = 4 * 148;
 
 template <int DT, int C, ShortBuild BUILD>
-__global__ void __launch_bounds__(kShortThreads, 4) qattn_short_kernel(AttnArgs a, int n_ctiles) {
+__global__ void __launch_bounds__(kShortThreads, BUILD == kNoUpdate ? 8 : 4) qattn_short_kernel(AttnArgs a, int n_ctiles) {
     __shared__ __align__(16) float q_s[C][2 * kHalfStride];
     __shared__ __align__(16) float qg_s[C][2 * 36];
     __shared__ __align__(16) float red_s[4][C][kHeadDim];       // prologue: down projections of the query update; end: the warps' sums
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(kShortThreads, 4) qattn_short_kernel(AttnArgs 
     if (BUILD == kRank32) {
         const int32_t li = adapter_of(a, b, tid);
         if (li >= 0) lora_update_small<32, C>(a, li, b, hkv, Gq, col0, ncols, red_s[0][0], warp, lane, qv);
-    } else if (a.lora.x) {
+    } else if (BUILD == kAnyUpdate && a.lora.x) {
         lora_update<C>(a, b, hkv, Gq, col0, ncols, red_s[0], tid, warp, lane, qv);
     }
     if (a.rotate_q) wht128_warp(qv, lane);
@@ -382,8 +385,9 @@ bool short_eligible(const AttnArgs& a) {
     return a.S <= 4096 && a.B * a.Hkv * cols <= 0x7fffffffLL;
 }
 
-// Fewer than 128 keys and 1,024 rows: always (the fp32 kernel for calls that were never given to fp16 operands; the
-// lane-per-key kernel takes 8-20 us on them, this one 3.5-9).  Otherwise it competes with the warp-level tensor-core kernel,
+// Fewer than 128 keys and 1,024 rows: always (calls that were never given to fp16 operands; the lane-per-key kernel takes
+// 8 to 20 us on them, this one 3.3 to 12.6, the most with 127 users x 8 heads x 127 keys, where the tensor-core kernel takes
+// 12.5).  Otherwise it competes with the warp-level tensor-core kernel,
 // which costs 8 to 10 us before its first key but less per key: measured (device time, one column per kv head) 8 CTAs x 4 passes of
 // 64 keys 6.0 us against 12, x 8 passes 9.4 against 14, 512 x 2 passes 8.4 against 9.5, 512 x 4 13.3 against 13, 2,048 x 2 23.7
 // against 20.5; four columns: 32 CTAs x 4 passes 11.8 against 14, x 8 20 against 16, 512 x 1 9.7 against 10, 512 x 2 14.4 against 11.
@@ -409,6 +413,8 @@ static int32_t launch_short_c(const AttnArgs& a, cudaStream_t st) {
     if (L.x && a.T == 1 && L.hidden == 128 && L.rank == 32 &&
         ((reinterpret_cast<uintptr_t>(L.x) | reinterpret_cast<uintptr_t>(L.a) | reinterpret_cast<uintptr_t>(L.b)) & 15) == 0)
         return launch_short_build<DT, C, kRank32>(a, st);
+    if constexpr (C == 1)
+        if (!L.x && a.B * a.Hkv > kFourPerSm) return launch_short_build<DT, 1, kNoUpdate>(a, st);
     return launch_short_build<DT, C, kAnyUpdate>(a, st);
 }
 

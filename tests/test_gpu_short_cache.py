@@ -95,6 +95,21 @@ def test_short_cache_query_update(dev, Hq, Hkv, T, hid, rank, monkeypatch):
     assert torch.equal(bad, fa.omni_attn(q.to(dev), *cache, user_id=6, n_splits=1))
 
 
+@pytest.mark.parametrize("S", [1, 17, 64, 127])
+def test_more_ctas_than_four_per_sm(dev, S):
+    """One column and 600 CTAs: the build for eight CTAs per SM, which the default route takes too."""
+    fa = attn_mod()
+    kn, kq, kr, vn, cb, gen = make_cache(75, 8, S, seed=S, user_id=3)
+    q = torch.randn(75, 8, 1, 128, generator=gen).to(torch.float16)
+    d = to_dev(dev, q, kn, kq, kr, vn, cb)
+    lens = torch.randint(0, S + 1, (75,), generator=gen, dtype=torch.int32)
+    lens[0], lens[1] = S, 0
+    assert (fa.omni_attn(*d, user_id=3, n_splits=1).cpu() - orc.decode_attention(q, kn, kq, kr, vn, cb, 3)).abs().max() <= ATOL
+    few = [fa.omni_attn(*[x[b:b + 25] for x in d[:5]], d[5], user_id=3, seq_lens=lens[b:b + 25].to(dev), n_splits=1) for b in (0, 25, 50)]
+    many = fa.omni_attn(*d, user_id=3, seq_lens=lens.to(dev), n_splits=1)
+    assert (many - torch.cat(few)).abs().max() <= 1e-5 and not many[1].any()
+
+
 def test_rank_32_costs_little_more_than_rank_16(dev, monkeypatch):
     """All rows of a rank-32 update are requested ahead, as those of rank 16 (16 users x 8 heads x 50 keys: 5.5 us;
     with the general form 9.8)."""
