@@ -137,7 +137,8 @@ int32_t omni_qjl_reconstruct_bool(const uint8_t* signs, const float* norms, int6
  * [n_groups+1], first entry 0, last n_total, at least 16 samples per group).  `workspace`: device scratch of
  * omni_lloyd_max_workspace_bytes(n_total) bytes (fp64 prefix sums).  codebooks: device fp32 [n_groups][16];
  * iters_out: device int32 [n_groups] (iterations run) or NULL.  Means are formed in fp64 and rounded once, so
- * the result equals the reference's to a few fp32 ulps rather than bit for bit.                                */
+ * the result equals the reference's to a few fp32 ulps rather than bit for bit.  A group with an infinite or NaN
+ * sample gets a codebook that is not finite; the other groups' codebooks do not depend on it.                  */
 size_t  omni_lloyd_max_workspace_bytes(int64_t n_total);
 int32_t omni_lloyd_max_fit(const float* sorted, int64_t n_total, const int64_t* group_offsets, int32_t n_groups,
                            int32_t max_iters, double tol, void* workspace, size_t workspace_bytes,

@@ -210,13 +210,18 @@ __global__ void __launch_bounds__(kSortThreads) sort_scatter_kernel(const void* 
 
 static size_t aligned256(size_t n) { return (n + 255) & ~(size_t)255; }
 
+// The prefix sums run over all groups back to back, so they leave infinite and NaN samples out: in the sums they would turn
+// every later group's means into NaN.  The group that holds them adds them to the cells they fall into.
+__device__ __forceinline__ double finite_or_zero(float x) { return isfinite(x) ? (double)x : 0.0; }
+__device__ __forceinline__ double if_not_finite(float x) { return isfinite(x) ? 0.0 : (double)x; }
+
 // Pass 1: the fp64 sum of every chunk of kScanChunk samples.
 __global__ void __launch_bounds__(kScanThreads) chunk_sums_kernel(const float* x, int64_t n, double* chunk_sum) {
     const int64_t base = (int64_t)blockIdx.x * kScanChunk;
     double s = 0.0;
     for (int j = 0; j < kScanPerThread; ++j) {
         const int64_t i = base + (int64_t)j * kScanThreads + threadIdx.x;     // coalesced
-        if (i < n) s += (double)x[i];
+        if (i < n) s += finite_or_zero(x[i]);
     }
     double total;
     block_inclusive_scan(s, &total);
@@ -252,7 +257,8 @@ __global__ void __launch_bounds__(kScanThreads) write_prefix_kernel(const float*
     double s = 0.0;
 #pragma unroll
     for (int j = 0; j < kScanPerThread; ++j) {
-        v[j] = first + 32 * j < n ? x[first + 32 * j] : 0.f;
+        const float xj = first + 32 * j < n ? x[first + 32 * j] : 0.f;
+        v[j] = isfinite(xj) ? xj : 0.f;
         s += (double)v[j];
     }
 #pragma unroll
@@ -317,11 +323,18 @@ __global__ void __launch_bounds__(kLloydWarps * 32) lloyd_max_kernel(const float
     const int64_t lo = group_off[g], hi = group_off[g + 1], n = hi - lo;
     const int64_t per = n / kLevels;
     float* const cent = cent_s[c];
+    // sorted in ascending order, NaN last: the ends tell whether every sample is finite
+    const bool finite = isfinite(sorted[lo]) && isfinite(sorted[hi - 1]);
+    // a range's mean; its infinite or NaN samples lie at its ends
+    auto mean = [&](double sum, int64_t a, int64_t b) {
+        if (!finite) sum += if_not_finite(sorted[a]) + if_not_finite(sorted[b - 1]);
+        return (float)(sum / (double)(b - a));
+    };
     // equal-mass initialisation: the mean of each sixteenth of the sorted sample
     float mine = 0.f;
     if (lane < kLevels) {
         const int64_t a = lo + lane * per, b = a + per;
-        mine = (float)((prefix[b] - prefix[a]) / (double)per);
+        mine = mean(prefix[b] - prefix[a], a, b);
         cent[lane] = mine;
     }
     if (threadIdx.x < 2) {
@@ -329,8 +342,6 @@ __global__ void __launch_bounds__(kLloydWarps * 32) lloyd_max_kernel(const float
         bound_s[threadIdx.x][kLevels] = hi; pre_s[threadIdx.x][kLevels] = prefix[hi];
     }
     __syncthreads();
-    // sorted in ascending order, NaN last: the ends tell whether every sample is finite
-    const bool finite = isfinite(sorted[lo]) && isfinite(sorted[hi - 1]);
     int64_t at = lo + (c + 1) * per, step = 0;                       // this warp's boundary and its last move
     int steps = 0;
     for (int64_t span = n; span > 0; span >>= 1) ++steps;            // enough halvings for a range of n + 1 positions
@@ -403,7 +414,7 @@ __global__ void __launch_bounds__(kLloydWarps * 32) lloyd_max_kernel(const float
         if (lane < kLevels) {
             const int64_t a = bound_s[buf][lane], b = bound_s[buf][lane + 1];
             if (b > a) {                                             // an empty cell keeps its centroid
-                const float fresh = (float)((pre_s[buf][lane + 1] - pre_s[buf][lane]) / (double)(b - a));
+                const float fresh = mean(pre_s[buf][lane + 1] - pre_s[buf][lane], a, b);
                 moved = fabsf(fresh - mine);
                 mine = fresh;
             }

@@ -40,3 +40,20 @@ def test_search_matches_assignment(kind, iters):
     got = calibrate_per_group([other.cuda(), x.cuda()], max_iters=iters).cpu()[1]
     assert (got - lloyd_iterations(x, iters)).abs().max() <= 2 * 2.0 ** -23 * float(x.abs().max())
 
+
+@pytest.mark.parametrize("bad", [float("inf"), -float("inf"), float("nan")])
+@pytest.mark.parametrize("first", [False, True])
+def test_groups_beside_one_that_is_not_finite(bad, first):
+    """A group with an infinite or NaN sample has no finite codebook; the other groups of the call get theirs as without it."""
+    from omnistack_rs_b200.quantization import calibrate_per_group
+    gen = torch.Generator().manual_seed(3)
+    groups = [torch.randn(n, generator=gen).cuda() for n in (5000, 300, 70000)]
+    spoilt = torch.randn(4000, generator=gen).cuda()
+    spoilt[17] = bad
+    alone = calibrate_per_group(groups, max_iters=40)
+    both = calibrate_per_group([spoilt] + groups if first else groups + [spoilt], max_iters=40)
+    assert not both[0 if first else 3].isfinite().all()
+    rest = both[1:] if first else both[:3]
+    # behind other samples the prefix sums of a group start at another value: their fp64 rounding, 2^-53 * 1e5 samples * 3, is far
+    # below an fp32 ulp of a mean, which it can still move across a rounding boundary, and the iterations carry that on
+    assert torch.equal(rest, alone) if not first else (rest - alone).abs().max() <= 1e-5
