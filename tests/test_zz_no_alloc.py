@@ -51,7 +51,7 @@ def _call(lib, name, q, kn, kq, kr, vn, cb, lens, n_splits, workspace=None):
     return status, out
 
 
-def test_noalloc_entry_matches_regular_entry_twice():
+def test_noalloc_entry_matches_regular_entry_twice(monkeypatch):
     from omnistack_rs_b200 import _lib
     assert torch.cuda.is_available(), "GPU tests need a CUDA device"
     dev = torch.device("cuda:0")
@@ -59,8 +59,11 @@ def test_noalloc_entry_matches_regular_entry_twice():
     assert lib.omni_qattn_noalloc_scratch_bytes() == 32 << 20
     with torch.cuda.device(dev):
         free_before = None
-        # the last case (100 keys, 2 splits) takes the lane-per-key kernel and the merge over the built-in scratch
-        for B, Hq, Hkv, S, n_splits, seed in ((5, 8, 4, 700, 6, 1), (3, 4, 2, 130, 3, 2), (2, 4, 2, 100, 2, 3)):
+        # the warp-level and the lane-per-key kernel, with the merge over the built-in scratch, and the short-cache kernel, which
+        # needs none of it
+        for B, Hq, Hkv, S, n_splits, seed, kernel in ((5, 8, 4, 700, 6, 1, "mma"), (3, 4, 2, 130, 3, 2, "mma"), (2, 4, 2, 100, 2, 3, "lane"),
+                                                      (2, 4, 2, 100, 2, 4, "short")):
+            monkeypatch.setenv("OMNI_QATTN_KERNEL", kernel)
             kn, kq, kr, vn, cb, gen = _cache(B, Hkv, S, seed)
             q = torch.randn(B, Hq, 2, 128, generator=gen).to(torch.bfloat16)
             lens = torch.randint(1, S + 1, (B,), generator=gen).to(torch.int32)
