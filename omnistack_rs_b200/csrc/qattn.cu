@@ -23,7 +23,7 @@ __global__ void __launch_bounds__(kAttnWarps * 32) qattn_lane_per_key_kernel(Att
         if (!__syncthreads_or(wide)) return;
     }
     const int wib = threadIdx.x >> 5;
-    lane_per_key_rows<DT>(a, scratch[wib], (int64_t)blockIdx.x * kAttnWarps + wib, (int64_t)gridDim.x * kAttnWarps);
+    lane_per_key_rows<DT, true>(a, scratch[wib], (int64_t)blockIdx.x * kAttnWarps + wib, (int64_t)gridDim.x * kAttnWarps);
 }
 
 // Merge the per-split partial states of one (user, head, token).  A CTA per output row; its warps take the splits

@@ -168,17 +168,58 @@ __device__ __forceinline__ void lora_up_rows(const LoraFold& L, const float* con
     }
 }
 
-// The update of one query row (lane-per-key kernel): both steps, then q += alpha * up.
-static __device__ __noinline__ void lora_fold_row(const LoraFold L, int64_t b, int T, int tq, int n_out, int o, int lane,
-                                                  int32_t* status, float (&qv)[4]) {
-    float d[4];
-    const int adapter = lora_down(L, b, T, tq, lane, d, status);
-    if (adapter < 0) return;
-    const float* const br[1] = {L.b + ((int64_t)adapter * n_out + o) * L.rank};
-    float up[1][4];
-    lora_up_rows<1>(L, br, d, up);
+// The update of one query row (lane-per-key code): the up projection takes each down-projected value as it comes, in the
+// order of the other forms, then q += alpha * up.
+__device__ __forceinline__ void lora_fold_row(const LoraFold& L, int64_t b, int T, int tq, int n_out, int o, int lane, int32_t* status, float (&qv)[4]) {
+    int32_t li = __ldg(L.idx + b);
+    if (li >= L.n_adapters) {
+        if (status && lane == 0) atomicMax(status, OMNI_STATUS_BAD_INDEX);
+        li = -1;
+    }
+    if (li < 0) return;
+    const float* xr = L.x + (b * T + tq) * (int64_t)L.hidden;
+    const float* am = L.a + (int64_t)li * L.rank * L.hidden;
+    const float* br = L.b + ((int64_t)li * n_out + o) * L.rank;
+    float up[4] = {0.f, 0.f, 0.f, 0.f};
+    int r = 0;
+    if (L.rank % 4 == 0 && (reinterpret_cast<uintptr_t>(L.b) & 15) == 0) {
+        // four rows at a time; the common hidden size has all their loads in flight at once
+        const bool one_pass = L.hidden == 128 && ((reinterpret_cast<uintptr_t>(xr) | reinterpret_cast<uintptr_t>(am)) & 15) == 0;
+        float4 xv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (one_pass) xv = __ldg(reinterpret_cast<const float4*>(xr) + lane);
+        for (; r < L.rank; r += 4) {
+            float4 w[4];
+            float d[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) qv[i] = fmaf(up[0][i], L.alpha, qv[i]);
+            for (int i = 0; i < 4; ++i) w[i] = __ldg(reinterpret_cast<const float4*>(br + (int64_t)i * L.rank + r));
+            if (one_pass) {
+                float4 av[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) av[j] = __ldg(reinterpret_cast<const float4*>(am + (int64_t)(r + j) * 128) + lane);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    float v = 0.f;
+                    v = fmaf(xv.x, av[j].x, v); v = fmaf(xv.y, av[j].y, v); v = fmaf(xv.z, av[j].z, v); v = fmaf(xv.w, av[j].w, v);
+                    d[j] = warp_sum(v);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) d[j] = lora_down_row(xr, am + (int64_t)(r + j) * L.hidden, L.hidden, lane);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                up[i] = fmaf(d[0], w[i].x, up[i]); up[i] = fmaf(d[1], w[i].y, up[i]);
+                up[i] = fmaf(d[2], w[i].z, up[i]); up[i] = fmaf(d[3], w[i].w, up[i]);
+            }
+        }
+    }
+    for (; r < L.rank; ++r) {
+        const float d = lora_down_row(xr, am + (int64_t)r * L.hidden, L.hidden, lane);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) up[i] = fmaf(d, __ldg(br + (int64_t)i * L.rank + r), up[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) qv[i] = fmaf(up[i], L.alpha, qv[i]);
 }
 
 // The common small case with every extent known at compile time, so that the loads of a step are all issued before

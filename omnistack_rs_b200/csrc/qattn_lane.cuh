@@ -1,16 +1,21 @@
 // The fp32 lane-per-key attention of one warp: the lane-per-key kernel (qattn.cu) and, for codebooks that the fp16 tables
 // cannot hold, the warp-level tensor-core kernel (qattn_mma.cu) run it over their share of the work units.
 //
-// Work unit: one warp per (user, query head, query token, key split).  Lane l walks
-// keys l, l+32, ... of its split with a private online-softmax state (max, sum, 128
-// accumulators); nothing crosses lanes until the final merge.  K and V are dequantised
-// in registers by a 16-entry codebook lookup in shared memory (16 words occupy 16
-// distinct banks, so any access pattern is conflict-free).  The QJL part of K is
+// Work unit: one warp per (user, query head, query token, key split), 32 keys at a time.  Scores: lane = key, its K row
+// dequantised in registers by a 16-entry codebook lookup in shared memory (16 words occupy 16 distinct banks, so any access
+// pattern is conflict-free) and multiplied with the query row from shared memory.  Output: lane = 8 dims of one key of each of
+// the 16 pairs of the pair layout, so a V row is read as consecutive words and eight accumulators suffice.  The QJL part of K is
 // applied as a score correction  norm * c * sum_i s_i (q . g_i)  with the 64 values
 // (q . g_i) computed once per work unit -- the same algebra as the reference kernel
 // (kernels/fused_attention.py:198-213, 260-276) but with G seeded per (user, kv head)
 // exactly as the codec does (kernels/quantize.py:583), which is what the reference's
 // CPU path (kernels/fused_attention.py:435-466) computes.
+//
+// What bounds it: the shared-memory pipe (256 codebook lookups per 32 keys).  The same lane = key for the output took 128
+// accumulators per lane, 168 registers and a butterfly over 128 values per work unit: 64 users x 8 heads x 2,048 keys 112.6 us
+// against 104.5, 32 x 32 x 300 41.2 against 37.9, and called from the warp-level kernel it cost that kernel spills.  Error against
+// fp64 (relative 2-norm, 4 users x 32 heads x 32,768 keys, centroids to 11): 7.3e-7, with per-lane maxima and one serial sum
+// per dot product 1.9e-6.
 #pragma once
 #include "qattn.cuh"
 
@@ -24,8 +29,11 @@ struct LaneScratch {                 // one warp's shared memory
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];\n" :: "l"(p)); }
 
+// Key pairs of the pair layout, in order: (0,3), (1,2), (4,7), (5,6) of every group of eight; the second key is the first ^ 3.
+__device__ __forceinline__ constexpr int pair_first(int j) { return 8 * (j >> 2) + (j & 1) + 2 * (j & 2); }
+
 // Work units first, first + stride, ... of B * Hq * T * n_splits.
-template <int DT>
+template <int DT, bool LORA>
 __device__ __forceinline__ void lane_per_key_rows(const AttnArgs& a, LaneScratch& sc, int64_t first, int64_t stride) {
     const int lane = threadIdx.x & 31;
     const int64_t n_work = a.B * a.Hq * a.T * a.n_splits;
@@ -41,9 +49,8 @@ __device__ __forceinline__ void lane_per_key_rows(const AttnArgs& a, LaneScratch
     // ---- prologue: query, codebook, q . g_i ------------------------------------
     float qv[4];
     Elem<DT>::load4(a.q, qrow * kHeadDim + 4 * lane, qv);
-    if (a.lora.x) {                                   // per-user low-rank update of the query row
+    if (LORA && a.lora.x)                             // per-user low-rank update of the query row
         lora_fold_row(a.lora, b, a.T, (int)(qrow % a.T), a.Hq * kHeadDim, hq * kHeadDim + 4 * lane, lane, a.status, qv);
-    }
     if (a.rotate_q) wht128_warp(qv, lane);
     *reinterpret_cast<float4*>(&sc.q[4 * lane]) = make_float4(qv[0], qv[1], qv[2], qv[3]);
     {
@@ -85,133 +92,119 @@ __device__ __forceinline__ void lane_per_key_rows(const AttnArgs& a, LaneScratch
     const int64_t slot = a.cache_slots ? (int64_t)a.cache_slots[b] : b;
     const int64_t base_row = slot * a.ks_b + (int64_t)hkv * a.ks_h;
 
-    float m = -INFINITY, l = 0.f;
-    float O[kHeadDim];
-#pragma unroll
-    for (int d = 0; d < kHeadDim; ++d) O[d] = 0.f;
+    const int64_t paired = a.v_paired ? (len & ~(int64_t)7) : 0;       // keys below this are stored pair-wise
     const float* qs = sc.q;
     const float* cbs = sc.cb;
+    const int half = lane >> 4, w = lane & 15;
+    float m = -INFINITY, l = 0.f, O[8];                // m: the same in every lane; l: of this lane's keys
+#pragma unroll
+    for (int n = 0; n < 8; ++n) O[n] = 0.f;
 
-    for (int64_t k = s0 + lane; k < s1; k += 32) {
-        const int64_t row = base_row + k;
+    // the K row, sign bytes and norm of this lane's key among 32 (the last key where there are fewer); the next 32 keys' are
+    // fetched as soon as the scores no longer need these
+    uint4 kw[4];
+    uint2 sb = make_uint2(0u, 0u);
+    float nrm = 0.f;
+    auto fetch_k = [&](int64_t k0) {
+        const int64_t row = base_row + (k0 + lane < s1 ? k0 + lane : s1 - 1);
         const uint4* kp = reinterpret_cast<const uint4*>(a.k_nib + row * kNibBytes);
-        // This key's sign bytes, norm and V row are needed one after the other further down: on a cold cache that is
-        // three memory latencies in a row, so they are requested now, together with the K and V rows of the lane's
-        // next key (a V row in the pair layout lies in this key's row and its partner's: the same 512-byte group).
-        prefetch_l2(a.v_nib + row * kNibBytes);
-        if (a.v_paired && k < (len & ~(int64_t)7)) prefetch_l2(a.v_nib + (base_row + (k ^ 3)) * kNibBytes);
-        if (a.with_qjl) { prefetch_l2(a.k_qjl + row * kQjlBytes); prefetch_l2(a.k_norms + row); }
-        if (k + 32 < s1) { prefetch_l2(a.k_nib + (row + 32) * kNibBytes); prefetch_l2(a.v_nib + (row + 32) * kNibBytes); }
-        float dot = 0.f;
 #pragma unroll
-        for (int c4 = 0; c4 < 4; ++c4) {
-            const uint4 wv = __ldg(kp + c4);
-            const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-            for (int wi = 0; wi < 4; ++wi) {
-                const float4 qa = *reinterpret_cast<const float4*>(qs + c4 * 32 + wi * 8);
-                const float4 qb = *reinterpret_cast<const float4*>(qs + c4 * 32 + wi * 8 + 4);
-                const uint32_t w = ww[wi];
-                dot = fmaf(qa.x, cbs[w & 15], dot);
-                dot = fmaf(qa.y, cbs[(w >> 4) & 15], dot);
-                dot = fmaf(qa.z, cbs[(w >> 8) & 15], dot);
-                dot = fmaf(qa.w, cbs[(w >> 12) & 15], dot);
-                dot = fmaf(qb.x, cbs[(w >> 16) & 15], dot);
-                dot = fmaf(qb.y, cbs[(w >> 20) & 15], dot);
-                dot = fmaf(qb.z, cbs[(w >> 24) & 15], dot);
-                dot = fmaf(qb.w, cbs[(w >> 28) & 15], dot);
-            }
-        }
-        float score = dot * a.scale;
+        for (int c = 0; c < 4; ++c) kw[c] = __ldg(kp + c);
         if (a.with_qjl) {
-            const uint2 sb = __ldg(reinterpret_cast<const uint2*>(a.k_qjl + row * kQjlBytes));
-            const float nrm = __ldg(a.k_norms + row);
-            float corr = 0.f;
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-                const float g0 = sc.qg[i], g1 = sc.qg[i + 32];
-                corr += ((sb.x >> i) & 1u) ? g0 : -g0;
-                corr += ((sb.y >> i) & 1u) ? g1 : -g1;
-            }
-            score = fmaf(nrm, corr, score);
+            sb = __ldg(reinterpret_cast<const uint2*>(a.k_qjl + row * kQjlBytes));
+            nrm = __ldg(a.k_norms + row);
         }
-        const float m_new = fmaxf(m, score);
-        const float p = expf(score - m_new);
-        if (m_new > m) {
-            const float alpha = expf(m - m_new);
-            l *= alpha;
+    };
+    if (s0 < s1) fetch_k(s0);
+
+    for (int64_t k0 = s0; k0 < s1; k0 += 32) {
+        // ---- the lane's word of one key of every pair, used after the scores ----
+        const int n_keys = s1 - k0 < 32 ? (int)(s1 - k0) : 32;
+        uint32_t vw[16];
 #pragma unroll
-            for (int d = 0; d < kHeadDim; ++d) O[d] *= alpha;
-            m = m_new;
+        for (int j = 0; j < 16; ++j) {
+            const int key = pair_first(j) ^ (3 * half);
+            vw[j] = __ldg(reinterpret_cast<const uint32_t*>(a.v_nib + (base_row + k0 + (key < n_keys ? key : n_keys - 1)) * kNibBytes) + w);
         }
-        l += p;
-        if (a.v_paired && k < (len & ~(int64_t)7)) {
-            // pair layout: this key's even-d nibbles sit in the row of the pair's first key, its odd-d nibbles in
-            // the row of the second (pairs (0,3), (1,2), (4,7), (5,6) of a group of eight: partner = key ^ 3), in
-            // the low nibbles when this key is the first of the pair, else in the high ones
-            const int64_t first = (k & 2) ? (k ^ 3) : k;
-            const int sh = (k & 2) ? 4 : 0;
-            const uint4* xp = reinterpret_cast<const uint4*>(a.v_nib + (base_row + first) * kNibBytes);
-            const uint4* yp = reinterpret_cast<const uint4*>(a.v_nib + (base_row + (first ^ 3)) * kNibBytes);
+        if (k0 + 32 + lane < s1) prefetch_l2(a.v_nib + (base_row + k0 + 32 + lane) * kNibBytes);
+        // ---- scores: lane = key ----
+        float dot[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-                const uint4 xv = __ldg(xp + c4), yv = __ldg(yp + c4);
-                const uint32_t xw[4] = {xv.x, xv.y, xv.z, xv.w}, yw[4] = {yv.x, yv.y, yv.z, yv.w};
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t ww[4] = {kw[c].x, kw[c].y, kw[c].z, kw[c].w};
 #pragma unroll
-                for (int wi = 0; wi < 4; ++wi) {
+            for (int i = 0; i < 4; ++i) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int d = c4 * 32 + wi * 8 + 2 * i;
-                        O[d] = fmaf(p, cbs[(xw[wi] >> (8 * i + sh)) & 15], O[d]);
-                        O[d + 1] = fmaf(p, cbs[(yw[wi] >> (8 * i + sh)) & 15], O[d + 1]);
-                    }
-                }
-            }
-        } else {
-            const uint4* vp = reinterpret_cast<const uint4*>(a.v_nib + row * kNibBytes);
-#pragma unroll
-            for (int c4 = 0; c4 < 4; ++c4) {
-                const uint4 wv = __ldg(vp + c4);
-                const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
-#pragma unroll
-                for (int wi = 0; wi < 4; ++wi) {
-                    const uint32_t w = ww[wi];
-#pragma unroll
-                    for (int n = 0; n < 8; ++n)
-                        O[c4 * 32 + wi * 8 + n] = fmaf(p, cbs[(w >> (4 * n)) & 15], O[c4 * 32 + wi * 8 + n]);
+                for (int h = 0; h < 2; ++h) {
+                    const float4 q4 = *reinterpret_cast<const float4*>(qs + c * 32 + i * 8 + 4 * h);
+                    dot[0] = fmaf(q4.x, cbs[(ww[i] >> (16 * h)) & 15u], dot[0]);
+                    dot[1] = fmaf(q4.y, cbs[(ww[i] >> (16 * h + 4)) & 15u], dot[1]);
+                    dot[2] = fmaf(q4.z, cbs[(ww[i] >> (16 * h + 8)) & 15u], dot[2]);
+                    dot[3] = fmaf(q4.w, cbs[(ww[i] >> (16 * h + 12)) & 15u], dot[3]);
                 }
             }
         }
+        float score = ((dot[0] + dot[1]) + (dot[2] + dot[3])) * a.scale;
+        if (a.with_qjl) {
+            float corr[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int i = 0; i < 32; i += 4) {
+                const float4 ga = *reinterpret_cast<const float4*>(&sc.qg[i]), gb = *reinterpret_cast<const float4*>(&sc.qg[i + 32]);
+                const float g0[4] = {ga.x, ga.y, ga.z, ga.w}, g1[4] = {gb.x, gb.y, gb.z, gb.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    corr[e & 1] += ((sb.x >> (i + e)) & 1u) ? g0[e] : -g0[e];
+                    corr[2 + (e & 1)] += ((sb.y >> (i + e)) & 1u) ? g1[e] : -g1[e];
+                }
+            }
+            score = fmaf(nrm, (corr[0] + corr[1]) + (corr[2] + corr[3]), score);
+        }
+        if (k0 + 32 < s1) fetch_k(k0 + 32);
+        if (lane >= n_keys) score = -INFINITY;
+        const float m_new = fmaxf(m, warp_max(score));
+        const float p = expf(score - m_new), alpha = expf(m - m_new);
+        m = m_new;
+        l = fmaf(l, alpha, p);
+        // ---- output: lane = 8 dims of one key of a pair; summed over the 32 keys first, then added to the running sums ----
+        float acc[8];
+#pragma unroll
+        for (int n = 0; n < 8; ++n) acc[n] = 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (8 * (j >> 2) >= n_keys) break;
+            const float pj = __shfl_sync(kFullMask, p, pair_first(j) ^ (3 * half));
+            uint32_t x = vw[j];
+            if (k0 + 8 * (j >> 2) < paired) {          // (X: even dims of both keys, Y: odd dims) -> this key's word
+                const uint32_t o = __shfl_xor_sync(kFullMask, x, 16);
+                x = half ? ((o >> 4) & 0x0F0F0F0Fu) | (x & 0xF0F0F0F0u) : (x & 0x0F0F0F0Fu) | ((o & 0x0F0F0F0Fu) << 4);
+            }
+#pragma unroll
+            for (int n = 0; n < 8; ++n) acc[n] = fmaf(pj, cbs[(x >> (4 * n)) & 15u], acc[n]);
+        }
+#pragma unroll
+        for (int n = 0; n < 8; ++n) O[n] = fmaf(O[n], alpha, acc[n]);
     }
 
-    // ---- merge the 32 lane states ------------------------------------------------
-    const float m_w = warp_max(m);
-    const float f = (m == -INFINITY) ? 0.f : expf(m - m_w);
-    const float l_w = warp_sum(l * f);
+    // ---- add up the two halves; lane = dims 4 lane .. 4 lane + 3 ------------------------------------------------
+    const float l_w = warp_sum(l);
 #pragma unroll
-    for (int d = 0; d < kHeadDim; ++d) O[d] *= f;
-    // butterfly reduce-scatter: afterwards O[0..3] hold dims 4*lane .. 4*lane+3
+    for (int n = 0; n < 8; ++n) O[n] += __shfl_xor_sync(kFullMask, O[n], 16);
+    float o[4];
 #pragma unroll
-    for (int half = 64, mk = 16; half >= 4; half >>= 1, mk >>= 1) {
-        const bool upper = (lane & mk) != 0;
-#pragma unroll
-        for (int j = 0; j < half; ++j) {
-            const float send = upper ? O[j] : O[j + half];
-            const float keep = upper ? O[j + half] : O[j];
-            O[j] = keep + __shfl_xor_sync(kFullMask, send, mk);
-        }
+    for (int k = 0; k < 4; ++k) {
+        const float lo = __shfl_sync(kFullMask, O[k], lane >> 1), hi = __shfl_sync(kFullMask, O[k + 4], lane >> 1);
+        o[k] = (lane & 1) ? hi : lo;
     }
     if (a.n_splits == 1) {
-        float o[4];
         const float inv = l_w > 0.f ? 1.f / l_w : 0.f;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) o[k] = O[k] * inv;
+        for (int k = 0; k < 4; ++k) o[k] *= inv;
         if (a.unrotate_out) wht128_warp(o, lane);
         *reinterpret_cast<float4*>(a.out + qrow * kHeadDim + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
     } else {
-        float* w = a.ws + work * kWsStride;
-        *reinterpret_cast<float4*>(w + 4 * lane) = make_float4(O[0], O[1], O[2], O[3]);
-        if (lane == 0) { w[128] = m_w; w[129] = l_w; }
+        float* ws = a.ws + work * kWsStride;
+        *reinterpret_cast<float4*>(ws + 4 * lane) = make_float4(o[0], o[1], o[2], o[3]);
+        if (lane == 0) { ws[128] = m; ws[129] = l_w; }
     }
     __syncwarp();                      // the next unit overwrites this warp's query row in shared memory
     }

@@ -28,7 +28,8 @@
 // read of a stage is conflict free under the 64-byte swizzle.
 //
 // Work distribution.  Persistent grid, one CTA per SM.  Calls without key splits assign items statically (equal
-// sizes); split-K calls draw tickets from a counter in the workspace so ragged cache lengths stay balanced.
+// sizes); split-K calls with more items than warps draw tickets from a counter in the workspace, so ragged cache lengths
+// stay balanced.
 #include "qattn.cuh"
 #include "qattn_lane.cuh"
 #include <cuda.h>
@@ -681,10 +682,12 @@ __device__ __forceinline__ void ring_consumed(Ring& r) {
     --r.in_flight;
 }
 
-// Out of line: inlined, its 128 accumulators would take part in the register allocation of the main loop.
-template <int DT>
+// Out of line: inlined, it cost calls that do not need it up to 2 %, and up to 8 % with the query update.  What it calls decides
+// how the main loop's registers are assigned: keeping the arguments of its key loop in registers, or fetching the K rows later,
+// makes it 2 to 5 % faster and one-column calls that do not need it 1 to 3 % slower.
+template <int DT, bool LORA>
 __device__ __noinline__ void serve_in_fp32(const AttnArgs& a, LaneScratch& sc, int64_t first, int64_t stride) {
-    lane_per_key_rows<DT>(a, sc, first, stride);
+    lane_per_key_rows<DT, LORA>(a, sc, first, stride);
 }
 
 template <int DT, bool QJL, bool ONECOL, bool VPAIR, bool LORA>
@@ -707,15 +710,17 @@ qattn_mma_kernel(const __grid_constant__ AttnArgs a, int64_t n_items, const __gr
     const uint32_t my_off = (uint32_t)warp < n_front ? (uint32_t)warp * kWarpBlockBytes
                                                      : lut_off + kLutSpan + ((uint32_t)warp - n_front) * kWarpBlockBytes;
     {
-        // a codebook the fp16 table cannot hold to the error budget: the whole grid serves the call in fp32 instead
+        // a codebook the fp16 table cannot hold to the error budget: the whole grid serves the call in fp32 instead, the work
+        // units going round the CTAs first
         const int n_cb = a.cb_per_head ? a.Hkv * 16 : 16;
         bool wide = false;
         for (int i = threadIdx.x; i < n_cb; i += blockDim.x) wide = wide || centroid_is_wide(__ldg(a.codebooks + i));
         if (__syncthreads_or(wide)) {
             const int64_t cta = blockIdx.x + (int64_t)gridDim.x * blockIdx.y, ctas = (int64_t)gridDim.x * gridDim.y;
-            serve_in_fp32<DT>(a, reinterpret_cast<LaneScratch*>(smem)[warp], cta * kMmaWarps + warp, ctas * kMmaWarps);
+            serve_in_fp32<DT, LORA>(a, reinterpret_cast<LaneScratch*>(smem)[warp], warp * ctas + cta, ctas * kMmaWarps);
             return;
         }
+        if (a.cb_per_head && cb_head >= a.Hkv) return;       // SMs beyond the heads' share: they only help in fp32
     }
     const float lut_scale = lut_scale_of(a.codebooks + (a.cb_per_head ? cb_head * 16 : 0));
     const float inv_lut = 1.f / lut_scale;
@@ -1103,6 +1108,9 @@ static int32_t launch_mma_t(const AttnArgs& args, cudaStream_t st) {
         gy = 1;
     }
     if (ctas > items) ctas = items;                 // few items: one per CTA, spread over the SMs
+    // the SMs that this leaves idle take part when the codebooks turn out to be wide (1 user x 80 heads x 4,096 keys: 65 us on
+    // 80 SMs, 47 on all)
+    if (a.cb_per_head && gy < (unsigned)(sms / ctas)) gy = (unsigned)(sms / ctas);
     // ticket counters: not needed when every item has a warp of its own; cleared by the preparation launch when there is
     // one, by a memset node otherwise
     if (items <= ctas * kMmaWarps) a.work_counter = nullptr;
