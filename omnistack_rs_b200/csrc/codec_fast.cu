@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(kFqWarps * 32, 2) fast_quantize_kernel(const _
     // The 8-token groups of all (user, head) pairs, in order, are dealt out in equal consecutive shares, one per warp of the
     // grid: a warp's share may begin and end inside a pair.  A whole pair per warp left the last round of a large call
     // mostly empty and all but 8 warps of a one-user call idle: K and V of 1,024 users x 8 heads x 256 tokens (3.46 pairs
-    // per warp, so 4 rounds) 989 us against 862 us now, 256 x 8 x 203 fp32 rows with their rotation 202 against 187 us.
+    // per warp, so 4 rounds) 989 us against 862 us, 256 x 8 x 203 fp32 rows with their rotation 202 against 187 us.
     const int T = (int)a.T;                                          // fast_quantize_eligible: groups and tokens fit 32 bits
     const uint32_t gpp = (uint32_t)(T + 7) >> 3;                     // groups of one pair
     uint32_t gi, last;

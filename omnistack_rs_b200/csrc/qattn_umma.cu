@@ -26,7 +26,7 @@
 //
 // Covers: V rows in the reference or the pair layout, any S, ragged lengths, cache slots, split-K (static
 // assignment), rotation folding.  Wide codebooks (a centroid of magnitude 8 or
-// more) make the grid stand down exactly like the warp-level kernel; the fp32 kernel launched behind it takes over.
+// more) make the grid stand down; the fp32 kernel launched behind it takes over.
 #include "qattn.cuh"
 #include <mutex>
 #include <utility>

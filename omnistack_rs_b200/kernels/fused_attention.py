@@ -261,7 +261,7 @@ def _build_call(q, k_nibbles, k_qjl, k_norms, v_nibbles, codebooks, user_id, sca
 def _qattn(q, k_nibbles, k_qjl, k_norms, v_nibbles, codebooks, user_id, scale, with_qjl,
            seq_lens=None, cache_slots=None, rotate_q=False, unrotate_out=False, n_splits=None, lora=None,
            v_paired=False):
-    """One call of ``omni_qattn_decode_lora``; ``lora`` = (x, lora_a, lora_b, lora_indices, lora_alpha) or None.
+    """One call of ``omni_qattn_decode_call``; ``lora`` = (x, lora_a, lora_b, lora_indices, lora_alpha) or None.
     ``v_paired``: the V nibble rows are in the pair layout of :func:`pair_v_rows` (a resident cache's own format).
     Calls that repeat on the same cache tensors (a serving loop) reuse the checked and converted argument block of
     the first one; only the query, the LoRA inputs, the stream and the output are handled per call."""

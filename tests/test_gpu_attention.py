@@ -512,7 +512,7 @@ def test_dense_anchor_matches_oracle_and_packed_kernel(dev):
 def test_wide_codebook_with_peaked_softmax(dev, kernel_choice):
     """Centroids out to +-20 (an un-rotated cache with outlier channels) and queries aligned with single keys,
     so one key carries most of the softmax: fp16 centroids would be off by up to 2^-8 here.  Whichever kernel is
-    asked for, the call is served in fp32 (the tensor-core kernel stands down for such codebooks) and meets the
+    asked for, the call is served in fp32 (by the warp-level kernel's own grid for such codebooks) and meets the
     same 3e-3 as everywhere else.  Reference semantics: any fp32 codebook, kernels/quantize.py:620-636."""
     fa = attn_mod()
     g = load_golden("wide_codebook_attention.npz")
@@ -535,7 +535,7 @@ def test_wide_codebook_with_peaked_softmax(dev, kernel_choice):
     assert float(want.abs().max()) > 5.0
     got = fa.omni_attn(*to_dev(dev, qq, kn, kq, kr, vn, cb), user_id=3)
     assert (got.cpu() - want).abs().max() <= ATOL
-    # split-K: the tensor-core launch stands down, the fp32 kernel writes the partial states the combine launch merges
+    # split-K: the fp32 code writes the partial states the combine launch merges
     got = fa.omni_attn(*to_dev(dev, qq, kn, kq, kr, vn, cb), user_id=3, n_splits=4)
     assert (got.cpu() - want).abs().max() <= ATOL
 
